@@ -107,27 +107,26 @@ namespace {
 
 // Default tiling (the Python autotuner overrides it with measured choices): lanes per pose
 // so that each lane owns about 8 fit points -- enough pairwise work per lane to amortise
-// the per-step group reduction and Adam tail -- and start blocks that waste the fewest pose
-// slots.  Pharmacophore-only poses are tiny, so they get the narrowest groups.
-void auto_tile(int mode, int max_fit, int n_starts, int* lpp, int* chunks) {
-  int l = *lpp;
-  if (l <= 0) {
-    const int m = mode == FSS_MODE_PHARM ? 0 : max_fit;
-    l = m < 64 ? 4 : (m < 128 ? 8 : (m < 256 ? 16 : 32));
-  }
-  *lpp = l;
-  if (*chunks > 0) return;
-  const int max_poses = kMaxThreads / l;
+// the per-step group reduction and Adam tail -- and the start blocks choose_chunks picks.
+// Pharmacophore-only poses are tiny, so they get the narrowest groups.
+int auto_lanes(int mode, int max_fit) {
+  const int m = mode == FSS_MODE_PHARM ? 0 : max_fit;
+  return m < 64 ? 4 : (m < 128 ? 8 : (m < 256 ? 16 : 32));
+}
+
+// Start blocks with the fewest idle pose slots, in CTAs of at most kMaxThreads.
+int auto_chunks(int lpp, int n_starts) {
+  const int max_poses = kMaxThreads / lpp;
   int best_c = 1, best_waste = 1 << 30;
   for (int c = 1; c <= n_starts; ++c) {
     const int ppc = (n_starts + c - 1) / c;
     if (ppc > max_poses) continue;
-    const int warps = (ppc * l + 31) / 32;
-    const int waste = warps * 32 / l * c - n_starts;  // idle pose slots
+    const int warps = (ppc * lpp + 31) / 32;
+    const int waste = warps * 32 / lpp * c - n_starts;  // idle pose slots
     if (waste < best_waste) { best_waste = waste; best_c = c; }
     if (waste == 0) break;
   }
-  *chunks = best_c;
+  return best_c;
 }
 
 }  // namespace
@@ -212,22 +211,19 @@ int align_launch(const fss_align_desc* d, cudaStream_t st) {
   // automatic code variant: wide register tile for large clouds, roomy registers for small
   const int var = d->kernel_variant > 0 ? d->kernel_variant - 1
                   : pharm ? 0 : combo ? 2 : (maxM >= 64 ? 1 : 2);
-  int lpp = tc ? 32 : d->lanes_per_pose, chunks = d->chunks;
+  int lpp = tc ? 32 : d->lanes_per_pose;
   // the ESP comparison splits surface points over the lanes, so it sizes the lanes
-  auto_tile(d->mode, combo ? std::max(maxNs, maxMs) : shape ? maxM : maxMp, d->n_starts, &lpp,
-            &chunks);
-  if (chunks < 1 || chunks > d->n_starts)
+  if (lpp <= 0)
+    lpp = auto_lanes(d->mode, combo ? std::max(maxNs, maxMs) : shape ? maxM : maxMp);
+  if (lpp > 32)
+    return set_error(FSS_ERR_INVALID, "fss_align: lanes_per_pose must be 1, 2, 4, 8, 16 or 32");
+  if (d->chunks > d->n_starts)
     return set_error(FSS_ERR_INVALID, "fss_align: chunks must be in [1, n_starts]");
-  const int ppc = (d->n_starts + chunks - 1) / chunks;
-  const int threads = ((ppc * lpp + 31) / 32) * 32;
-  if (threads > kMaxThreads)
-    return set_error(FSS_ERR_INVALID, "fss_align: too many starts per CTA for lanes_per_pose");
-  // every start block must be non-empty
-  chunks = (d->n_starts + ppc - 1) / ppc;
+  const int fewest = d->chunks > 0 ? 0 : auto_chunks(lpp, d->n_starts);
 
   AlignParams p{};
   p.mode = d->mode; p.n_pairs = d->n_pairs; p.n_starts = d->n_starts; p.steps = d->steps;
-  p.chunks = chunks; p.n_items = d->n_pairs * chunks;
+  p.chunks = d->chunks;
   p.maxN = maxN; p.maxM = maxM; p.maxNp = maxNp; p.maxMp = maxMp;
   p.pair_ref = d->pair_ref; p.pair_fit = d->pair_fit; p.order = d->order;
   p.ref_pts = reinterpret_cast<const float4*>(d->ref_pts); p.ref_off = d->ref_off;
@@ -267,7 +263,7 @@ int align_launch(const fss_align_desc* d, cudaStream_t st) {
   p.counter = d->scratch;
 
   const size_t nb = ((size_t)maxN + 7) / 8;
-  const size_t smem = sizeof(float) * kColdFields * (size_t)threads +
+  const size_t smem =   // staged clouds; the launcher adds the parked state of its threads
       (acc == 2 ? sizeof(float2) * kTceF2PerBlock * nb + sizeof(float4) * maxM + 16
        : tc ? sizeof(float4) * (kMmaP4PerBlock * nb + maxM) +
                sizeof(float2) * (kMmaC2PerBlock + kMmaQ2PerBlock) * nb + 16
@@ -277,13 +273,13 @@ int align_launch(const fss_align_desc* d, cudaStream_t st) {
                sizeof(float2) * ((size_t)maxNa + maxMa) + 16);
   int rc;
   switch (d->mode) {
-    case FSS_MODE_SHAPE: rc = launch_align_shape(lpp, acc, var, p, threads, d->cta_per_sm, smem, st); break;
-    case FSS_MODE_ESP: rc = launch_align_esp(lpp, acc, var, p, threads, d->cta_per_sm, smem, st); break;
+    case FSS_MODE_SHAPE: rc = launch_align_shape(lpp, acc, var, p, fewest, d->cta_per_sm, smem, st); break;
+    case FSS_MODE_ESP: rc = launch_align_esp(lpp, acc, var, p, fewest, d->cta_per_sm, smem, st); break;
     case FSS_MODE_ESP_COMBO:
-      rc = launch_align_combo(lpp, var, p, threads, d->cta_per_sm, smem, st);
+      rc = launch_align_combo(lpp, var, p, fewest, d->cta_per_sm, smem, st);
       break;
     default:
-      rc = launch_align_pharm(d->mode, lpp, d->pharm_extended, p, threads, d->cta_per_sm, smem,
+      rc = launch_align_pharm(d->mode, lpp, d->pharm_extended, p, fewest, d->cta_per_sm, smem,
                               st);
       break;
   }

@@ -5,10 +5,10 @@
 
 namespace fss {
 
-int launch_align_combo(int lpp, int var, const AlignParams& prm, int threads, int cps,
+int launch_align_combo(int lpp, int var, const AlignParams& prm, int fewest, int cps,
                        size_t smem, cudaStream_t st) {
-  if (var == 2) return dispatch_lanes<FSS_MODE_ESP_COMBO, 2>(lpp, prm, threads, cps, smem, st);
-  return dispatch_lanes<FSS_MODE_ESP_COMBO, 0>(lpp, prm, threads, cps, smem, st);
+  if (var == 2) return dispatch_lanes<FSS_MODE_ESP_COMBO, 2>(lpp, prm, fewest, cps, smem, st);
+  return dispatch_lanes<FSS_MODE_ESP_COMBO, 0>(lpp, prm, fewest, cps, smem, st);
 }
 
 }  // namespace fss

@@ -288,15 +288,95 @@ __global__ void __launch_bounds__(kMaxThreads, AlignVariant<VAR>::kMinCtas)
   }
 }
 
+// Threads of a CTA that holds `poses` poses of one pair.
+inline int tile_threads(int poses, int lpp) { return (poses * lpp + 31) / 32 * 32; }
+
+// Start blocks of a pair when the caller leaves them to the library.  Results do not depend
+// on them.  `fewest` is the count with the fewest idle pose slots, in CTAs of up to
+// kMaxThreads; it is kept for short runs (under 8 steps: staging the pair is most of a block)
+// and for launches of less than two rounds of resident CTAs, where the largest pairs decide
+// the time and run faster the fewer other warps share their SM (256 pairs of 15-50 atoms, 4
+// lanes: 2.06 ms in 7-warp CTAs, 2.82 ms with all 1-warp CTAs resident at once).  Otherwise:
+//  * up to 4 warps an SM in all: 1-warp CTAs, so that a few pairs spread over the SMs (one pair
+//    of 30 atoms, 50 x 200, 4 lanes: 930 -> 672 us);
+//  * two rounds or more: the CTA of 1, 2 or 4 warps (or `fewest`) that keeps the most useful
+//    warps resident, (starts / pose slots) x resident warps -- the slots weigh idle lanes, the
+//    residency what registers and the staged clouds leave -- and of equals the smallest, whose
+//    warps wait least for their block's slowest pose (a lane per pose: the largest, which
+//    stages a pair least often).  256 surface pairs, 16 lanes: 104.2 -> 83.4 ms (5-warp ->
+//    2-warp CTAs); 16 384 shape + pharm pairs of 20 x 100, 8 lanes: 28.1 -> 26.9 ms; 4096 of
+//    50 x 200, 4 lanes: 39.1 -> 32.3 ms.
+template <class Kern>
+int choose_chunks(Kern kern, int lpp, const AlignParams& prm, int cta_per_sm, size_t smem_fixed,
+                  size_t smem_thread, int fewest) {
+  const int S = prm.n_starts;
+  if (prm.steps < 8) return fewest;
+  const int one_warp = (S + std::max(1, 32 / lpp) - 1) / std::max(1, 32 / lpp);
+  if ((double)prm.n_pairs * one_warp <= 4.0 * num_sms()) return one_warp;
+  int best = fewest;
+  double best_score = 0.0;
+  for (int c = 0; c < 4; ++c) {
+    const int warps = c > 0 ? 1 << (c - 1) : 0;
+    const int slots = c > 0 ? std::max(1, warps * 32 / lpp) : (S + fewest - 1) / fewest;
+    const int chunks = (S + slots - 1) / slots;
+    const int threads = tile_threads(std::min(slots, S), lpp);
+    if (threads > kMaxThreads) continue;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads,
+                                                      smem_fixed + smem_thread * threads) !=
+            cudaSuccess || occ <= 0) {
+      (void)cudaGetLastError();   // a size that does not fit is passed over
+      continue;
+    }
+    if (cta_per_sm > 0) occ = std::min(occ, cta_per_sm);
+    if ((double)prm.n_pairs * chunks < 2.0 * occ * num_sms()) {
+      if (c == 0) return fewest;
+      continue;
+    }
+    const double score = (double)S * lpp / ((double)chunks * threads) * occ * (threads / 32);
+    if (score > best_score * 1.001 ||
+        (score > best_score * 0.999 && (S + chunks - 1) / chunks < (S + best - 1) / best && lpp > 1)) {
+      best_score = score;
+      best = chunks;
+    }
+  }
+  return best;
+}
+
+// `fewest` > 0: the start blocks are chosen here (prm.chunks not set yet), `fewest` of them in
+// the fewest-idle-slots tiling; 0: prm.chunks is the caller's.
 template <int LPP, int MODE, int ACC, int VAR, int EXT = 0>
-int launch_align(const AlignParams& prm, int threads, int cta_per_sm, size_t smem,
+int launch_align(AlignParams prm, int fewest, int cta_per_sm, size_t smem_fixed,
                  cudaStream_t st) {
   auto kern = align_kernel<LPP, MODE, ACC, VAR, EXT>;
-  cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem);
+  const size_t smem_thread = sizeof(float) * kColdFields;
+  int optin = 0, dev = 0;
+  cudaError_t ce = cudaGetDevice(&dev);
+  if (ce == cudaSuccess)
+    ce = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaFuncAttributes fa{};
+  if (ce == cudaSuccess) ce = cudaFuncGetAttributes(&fa, kern);
+  // the tiling the caller asked for (or the one of the fewest idle slots) has to fit
+  const int first = fewest > 0 ? fewest : prm.chunks;
+  const int threads0 = tile_threads((prm.n_starts + first - 1) / first, LPP);
+  if (threads0 > kMaxThreads)
+    return set_error(FSS_ERR_INVALID, "fss_align: too many starts per CTA for lanes_per_pose");
+  const size_t limit = (size_t)optin - fa.sharedSizeBytes;
+  if (ce == cudaSuccess && smem_fixed + smem_thread * threads0 > limit)
+    ce = cudaErrorInvalidValue;
+  if (ce == cudaSuccess)
+    ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)std::min(smem_fixed + smem_thread * kMaxThreads, limit));
   if (ce != cudaSuccess)
     return set_error(FSS_ERR_CUDA, std::string("fss_align: shared-memory attribute: ") +
                                        cudaGetErrorString(ce));
+  if (fewest > 0)
+    prm.chunks = choose_chunks(kern, LPP, prm, cta_per_sm, smem_fixed, smem_thread, fewest);
+  const int ppc = (prm.n_starts + prm.chunks - 1) / prm.chunks;
+  const int threads = tile_threads(ppc, LPP);
+  prm.chunks = (prm.n_starts + ppc - 1) / ppc;   // every start block non-empty
+  prm.n_items = prm.n_pairs * prm.chunks;
+  const size_t smem = smem_fixed + smem_thread * threads;
   int occ = 0;
   ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem);
   if (ce != cudaSuccess || occ <= 0)
@@ -308,28 +388,28 @@ int launch_align(const AlignParams& prm, int threads, int cta_per_sm, size_t sme
 }
 
 template <int MODE, int VAR, int EXT = 0>
-int dispatch_lanes(int lpp, const AlignParams& prm, int threads, int cps, size_t smem,
+int dispatch_lanes(int lpp, const AlignParams& prm, int fewest, int cps, size_t smem,
                    cudaStream_t st) {
   switch (lpp) {
-    case 1: return launch_align<1, MODE, 0, VAR, EXT>(prm, threads, cps, smem, st);
-    case 2: return launch_align<2, MODE, 0, VAR, EXT>(prm, threads, cps, smem, st);
-    case 4: return launch_align<4, MODE, 0, VAR, EXT>(prm, threads, cps, smem, st);
-    case 8: return launch_align<8, MODE, 0, VAR, EXT>(prm, threads, cps, smem, st);
-    case 16: return launch_align<16, MODE, 0, VAR, EXT>(prm, threads, cps, smem, st);
-    case 32: return launch_align<32, MODE, 0, VAR, EXT>(prm, threads, cps, smem, st);
+    case 1: return launch_align<1, MODE, 0, VAR, EXT>(prm, fewest, cps, smem, st);
+    case 2: return launch_align<2, MODE, 0, VAR, EXT>(prm, fewest, cps, smem, st);
+    case 4: return launch_align<4, MODE, 0, VAR, EXT>(prm, fewest, cps, smem, st);
+    case 8: return launch_align<8, MODE, 0, VAR, EXT>(prm, fewest, cps, smem, st);
+    case 16: return launch_align<16, MODE, 0, VAR, EXT>(prm, fewest, cps, smem, st);
+    case 32: return launch_align<32, MODE, 0, VAR, EXT>(prm, fewest, cps, smem, st);
     default: return set_error(FSS_ERR_INVALID, "fss_align: lanes_per_pose must be 1, 2, 4, 8, 16 or 32");
   }
 }
 
 // Per-mode launchers (one translation unit each).  var: as AlignVariant; acc: 0 FP32 lanes,
 // 1 tensor-core sums, 2 tensor-core exponents (shape and ESP modes only).
-int launch_align_shape(int lpp, int acc, int var, const AlignParams& prm, int threads, int cps,
+int launch_align_shape(int lpp, int acc, int var, const AlignParams& prm, int fewest, int cps,
                        size_t smem, cudaStream_t st);
-int launch_align_esp(int lpp, int acc, int var, const AlignParams& prm, int threads, int cps,
+int launch_align_esp(int lpp, int acc, int var, const AlignParams& prm, int fewest, int cps,
                      size_t smem, cudaStream_t st);
 int launch_align_pharm(int mode, int lpp, int ext, const AlignParams& prm, int threads,
                        int cps, size_t smem, cudaStream_t st);
-int launch_align_combo(int lpp, int var, const AlignParams& prm, int threads, int cps,
+int launch_align_combo(int lpp, int var, const AlignParams& prm, int fewest, int cps,
                        size_t smem, cudaStream_t st);
 
 }  // namespace fss
