@@ -1,5 +1,5 @@
 // fss_align.cu -- host side of the fused alignment (validation, tiling, dispatch) and the
-// small helper kernels (per-pair argmax, self overlaps).  The fused kernel itself lives in
+// small helper kernels (per-pair argmax, shape self overlaps).  The fused kernel itself lives in
 // fss_align_kernel.cuh and is instantiated per mode in fss_align_<mode>.cu.
 #include <algorithm>
 #include <cmath>
@@ -58,35 +58,6 @@ __global__ void self_overlap_kernel(const Pts pts, const int* __restrict__ off,
   shape_pose<32, ESP>(sP, sQc, sB, n, n, threadIdx.x, R, -c.x, -c.y, -c.z, k, e, inv2k, acc);
   acc.group_sum<32>();
   if (threadIdx.x == 0) out[m] = acc.v * Kc;
-}
-
-template <int EXT>
-__global__ void pharm_self_kernel(const Pts anc, const Pts vec, const int* __restrict__ off,
-                                  int n_mol, int max_n, PharmTables tab, float* out) {
-  extern __shared__ __align__(16) float4 smem[];
-  __shared__ float red[96];
-  const int m = blockIdx.x;
-  const int o0 = off[m], n = off[m + 1] - o0;
-  if (n < 0 || n > max_n) {
-    if (threadIdx.x == 0) out[m] = __int_as_float(0x7fc00000);
-    return;
-  }
-  float4* sRA = smem;
-  float4* sRV = sRA + n;
-  float4* sFA = sRV + n;
-  float4* sFV = sFA + n;
-  const float3 c = block_centroid(anc + o0, n, red);
-  stage_ref_pharm(anc + o0, vec + o0, n, c, sRA, sRV);
-  stage_fit_pharm(anc + o0, vec + o0, n, sFA, sFV);
-  __syncthreads();
-  Rot R;
-#pragma unroll
-  for (int i = 0; i < 9; ++i) R.r[i] = (i % 4 == 0) ? 1.f : 0.f;
-  Moments acc;
-  acc.zero();
-  pharm_pose<32, EXT>(sRA, sRV, sFA, sFV, n, n, threadIdx.x, R, -c.x, -c.y, -c.z, tab, acc);
-  acc.group_sum<32>();
-  if (threadIdx.x == 0) out[m] = acc.v;
 }
 
 PharmTables make_pharm_tables(bool directional) {
@@ -323,25 +294,6 @@ int self_overlap_launch(const float* pts, const int32_t* off, int n_mol, int max
   }
   if (ce != cudaSuccess) return set_error(FSS_ERR_CUDA, std::string("fss_self_overlap: ") + cudaGetErrorString(ce));
   return check_launch("fss_self_overlap");
-}
-
-int pharm_self_launch(const float* anc, const float* vec, const int32_t* off, int n_mol, int max_n,
-                      int directional, int extended, int f16, float* out, cudaStream_t st) {
-  if (n_mol < 0 || !anc || !off || !out || (directional && !vec))
-    return set_error(FSS_ERR_INVALID, "fss_pharm_self_overlap: bad arguments");
-  if (extended < 0 || extended > 2 || (extended && !directional))
-    return set_error(FSS_ERR_INVALID, "fss_pharm_self_overlap: extended must be 0, 1 or 2 "
-                                      "(directional tables)");
-  if (max_n > kMaxPoints) return set_error(FSS_ERR_UNSUPPORTED, "fss_pharm_self_overlap: molecule too large");
-  if (n_mol == 0) return FSS_OK;
-  const size_t smem = sizeof(float4) * 4 * (size_t)max_n + 16;
-  auto kern = extended == 1 ? pharm_self_kernel<1>
-              : extended == 2 ? pharm_self_kernel<2> : pharm_self_kernel<0>;
-  cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (ce != cudaSuccess) return set_error(FSS_ERR_CUDA, std::string("fss_pharm_self_overlap: ") + cudaGetErrorString(ce));
-  kern<<<n_mol, 32, smem, st>>>(Pts(anc, f16), Pts(vec, f16), off, n_mol, max_n,
-                                make_pharm_tables(directional != 0), out);
-  return check_launch("fss_pharm_self_overlap");
 }
 
 }  // namespace fss
