@@ -1,7 +1,7 @@
 // fss_align_combo.cu -- instantiations of the fused alignment kernel for vol_and_surf_esp
 // (shape-steered pose, ShaEP ESP comparison in the tracked score).  Code variants: base and
 // the one-CTA/SM register budget (the shape channel works on small heavy-atom clouds).
-#include "fss_align_kernel.cuh"
+#include "fss_align_spread.cuh"
 
 namespace fss {
 

@@ -291,6 +291,16 @@ __global__ void __launch_bounds__(kMaxThreads, AlignVariant<VAR>::kMinCtas)
 // Threads of a CTA that holds `poses` poses of one pair.
 inline int tile_threads(int poses, int lpp) { return (poses * lpp + 31) / 32 * 32; }
 
+// Start blocks of a pair in CTAs of one warp, and whether a launch of them has at most 4 warps
+// to an SM: one for each scheduler.
+inline int one_warp_blocks(int starts, int lpp) {
+  const int slots = std::max(1, 32 / lpp);
+  return (starts + slots - 1) / slots;
+}
+inline bool spread_out(const AlignParams& prm, int lpp) {
+  return (double)prm.n_pairs * one_warp_blocks(prm.n_starts, lpp) <= 4.0 * num_sms();
+}
+
 // Start blocks of a pair when the caller leaves them to the library.  Results do not depend
 // on them.  `fewest` is the count with the fewest idle pose slots, in CTAs of up to
 // kMaxThreads; it is kept for short runs (under 8 steps: staging the pair is most of a block)
@@ -299,10 +309,10 @@ inline int tile_threads(int poses, int lpp) { return (poses * lpp + 31) / 32 * 3
 // lanes: 2.06 ms in 7-warp CTAs, 2.82 ms with all 1-warp CTAs resident at once).  Otherwise:
 //  * up to 4 warps an SM in all: 1-warp CTAs, so that a few pairs spread over the SMs (one pair
 //    of 30 atoms, 50 x 200, 4 lanes: 930 -> 672 us);
-//  * two rounds or more: the CTA of 1, 2 or 4 warps (or `fewest`) that keeps the most useful
-//    warps resident, (starts / pose slots) x resident warps -- the slots weigh idle lanes, the
-//    residency what registers and the staged clouds leave -- and of equals the smallest, whose
-//    warps wait least for their block's slowest pose (a lane per pose: the largest, which
+//  * two rounds or more: the CTA of 1, 2 or 4 warps (or `fewest`) with the largest
+//    (starts / pose slots) x (resident warps)^1/4 -- the slots weigh idle lanes; 12 resident
+//    warps instead of 10 (what the staged clouds leave) gave 4 % -- and of equals the smallest,
+//    whose warps wait least for their block's slowest pose (a lane per pose: the largest, which
 //    stages a pair least often).  256 surface pairs, 16 lanes: 104.2 -> 83.4 ms (5-warp ->
 //    2-warp CTAs); 16 384 shape + pharm pairs of 20 x 100, 8 lanes: 28.1 -> 26.9 ms; 4096 of
 //    50 x 200, 4 lanes: 39.1 -> 32.3 ms.
@@ -311,8 +321,7 @@ int choose_chunks(Kern kern, int lpp, const AlignParams& prm, int cta_per_sm, si
                   size_t smem_thread, int fewest) {
   const int S = prm.n_starts;
   if (prm.steps < 8) return fewest;
-  const int one_warp = (S + std::max(1, 32 / lpp) - 1) / std::max(1, 32 / lpp);
-  if ((double)prm.n_pairs * one_warp <= 4.0 * num_sms()) return one_warp;
+  if (spread_out(prm, lpp)) return one_warp_blocks(S, lpp);
   int best = fewest;
   double best_score = 0.0;
   for (int c = 0; c < 4; ++c) {
@@ -333,7 +342,8 @@ int choose_chunks(Kern kern, int lpp, const AlignParams& prm, int cta_per_sm, si
       if (c == 0) return fewest;
       continue;
     }
-    const double score = (double)S * lpp / ((double)chunks * threads) * occ * (threads / 32);
+    const double score = (double)S * lpp / ((double)chunks * threads) *
+                         std::pow((double)occ * (threads / 32), 0.25);
     if (score > best_score * 1.001 ||
         (score > best_score * 0.999 && (S + chunks - 1) / chunks < (S + best - 1) / best && lpp > 1)) {
       best_score = score;
@@ -345,11 +355,11 @@ int choose_chunks(Kern kern, int lpp, const AlignParams& prm, int cta_per_sm, si
 
 // `fewest` > 0: the start blocks are chosen here (prm.chunks not set yet), `fewest` of them in
 // the fewest-idle-slots tiling; 0: prm.chunks is the caller's.
-template <int LPP, int MODE, int ACC, int VAR, int EXT = 0>
-int launch_align(AlignParams prm, int fewest, int cta_per_sm, size_t smem_fixed,
-                 cudaStream_t st) {
-  auto kern = align_kernel<LPP, MODE, ACC, VAR, EXT>;
-  const size_t smem_thread = sizeof(float) * kColdFields;
+// parked: bytes of shared memory per thread beside the staged clouds.
+template <int LPP, class Kern>
+int launch_kernel(Kern kern, size_t parked, AlignParams prm, int fewest, int cta_per_sm,
+                  size_t smem_fixed, cudaStream_t st) {
+  const size_t smem_thread = parked;
   int optin = 0, dev = 0;
   cudaError_t ce = cudaGetDevice(&dev);
   if (ce == cudaSuccess)
@@ -385,6 +395,38 @@ int launch_align(AlignParams prm, int fewest, int cta_per_sm, size_t smem_fixed,
   const int grid = std::max(1, std::min(prm.n_items, occ * num_sms()));
   kern<<<grid, threads, smem, st>>>(prm);
   return check_launch("fss_align");
+}
+
+template <int LPP, int MODE, int GROUP, int EXT, bool ALONE>
+__global__ void spread_kernel(const AlignParams p);
+
+// spread_kernel (fss_align_spread.cuh) or align_kernel.  They give the same bits, so the faster
+// one is taken: spread_kernel from 4 lanes a pose on, where a lane has at most 16 fit points --
+// beyond that the pairwise loop hides the optimiser, and align_kernel's tiles of four are the
+// better loop (256 surfaces of 200-400 points, 16 lanes: 83.4 and 86.1 ms; 8 lanes, shape: 23.7
+// and 25.8 ms; 256 pairs of 15-50 atoms, 8 lanes: 1.77 and 1.56 ms).  align_kernel also keeps
+// the tensor-core paths and the variants whose rounding of the rotation is their own: 2 and 4,
+// and 1 for ESP at 32 lanes.
+template <int LPP, int MODE, int ACC, int VAR, int EXT = 0>
+int launch_align(const AlignParams& prm, int fewest, int cta_per_sm, size_t smem_fixed,
+                 cudaStream_t st) {
+  constexpr bool kSpread = LPP >= 4 && ACC == 0 && VAR != 1 && VAR != 3 &&
+                           !(LPP == 32 && MODE == FSS_MODE_ESP && VAR == 0);
+  if constexpr (kSpread) {
+    constexpr int kGroup = 2 * AlignVariant<VAR>::kJB2;
+    constexpr bool kOneChannel = MODE == FSS_MODE_SHAPE || MODE == FSS_MODE_ESP ||
+                                 MODE == FSS_MODE_ESP_COMBO;
+    if constexpr (LPP == 4 && kGroup == 4 && kOneChannel) {
+      if (spread_out(prm, LPP))
+        return launch_kernel<LPP>(spread_kernel<LPP, MODE, kGroup, EXT, true>, 0, prm, fewest,
+                                  cta_per_sm, smem_fixed, st);
+    }
+    if (prm.maxM <= 16 * LPP)
+      return launch_kernel<LPP>(spread_kernel<LPP, MODE, kGroup, EXT, false>, 0, prm, fewest,
+                                cta_per_sm, smem_fixed, st);
+  }
+  return launch_kernel<LPP>(align_kernel<LPP, MODE, ACC, VAR, EXT>, sizeof(float) * kColdFields,
+                            prm, fewest, cta_per_sm, smem_fixed, st);
 }
 
 template <int MODE, int VAR, int EXT = 0>

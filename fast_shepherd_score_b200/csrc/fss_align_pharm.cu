@@ -1,7 +1,7 @@
 // fss_align_pharm.cu -- instantiations of the fused alignment kernel for the modes with a
 // pharmacophore channel (pharm, shape + directional pharm, shape + colour).  Their poses are
 // small and tail-heavy, so only the base code variant is built.
-#include "fss_align_kernel.cuh"
+#include "fss_align_spread.cuh"
 
 namespace fss {
 

@@ -1,5 +1,5 @@
 // fss_align_shape.cu -- instantiations of the fused alignment kernel for the shape mode (FP32-lane variants and tensor-core sums).
-#include "fss_align_kernel.cuh"
+#include "fss_align_spread.cuh"
 
 namespace fss {
 
