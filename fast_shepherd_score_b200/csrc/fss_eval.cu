@@ -6,127 +6,185 @@
 #include <algorithm>
 #include <cmath>
 
-#include "fss_internal.cuh"
+#include "fss_align_spread.cuh"
 
 namespace fss {
 
+namespace {
+
+constexpr int kFewLanes = 8;   // lanes of a pharmacophore pose with a small stage
+
+// Component c (0: V, 1-3: dV/dt, 4-7: dV/dq) of pose `row`.
+__device__ __forceinline__ void eval_write(int c, float x, size_t row, int need_grad, float* V,
+                                           float* dQ, float* dT) {
+  if (c == 0) V[row] = x;
+  else if (need_grad && c < 4) dT[row * 3 + c - 1] = x;
+  else if (need_grad) dQ[row * 4 + c - 4] = x;
+}
+
+// Expanded reference point (stage_ref).
 template <bool ESP>
-__global__ void __launch_bounds__(32) overlap_eval_kernel(
+__device__ __forceinline__ void expand_point(float ax, float ay, float az, float ci, float k,
+                                             float e, float4* P, float2* Q) {
+  float w = -k * (ax * ax + ay * ay + az * az);
+  if (ESP) {
+    w = fmaf(-e * ci, ci, w);
+    *Q = make_float2(2.f * e * ci, 2.f * e * ci);
+  }
+  const float px = 2.f * k * ax, py = 2.f * k * ay, pz = 2.f * k * az;
+  P[0] = make_float4(px, px, py, py);
+  P[1] = make_float4(pz, pz, w, w);
+}
+
+}  // namespace
+
+// A pose to a CTA of one warp (atom clouds) or two (surfaces).  A surface is bound by the pairwise
+// loop's ex2 and FP32 and wants more warps than one per pose; an atom cloud by the instructions and
+// latency around a short loop, where a second warp, or several poses to a warp, gave nothing.  The
+// reduction halves the components with the lanes (LanePose), 13 shuffles for 40.  One B200, before
+// (a warp a pose, full butterflies) -> after: 1600 poses of 200-400 charged points 129 -> 87 us, 20
+// of them 72 -> 35; 12 800 poses of 15-50 atoms 20.3 -> 19.7, 100 of them 4.5 -> 4.2.
+template <bool ESP, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) overlap_eval_kernel(
     const float* __restrict__ A, const float* __restrict__ B, const float* __restrict__ CA,
     const float* __restrict__ CB, const float* __restrict__ q, const float* __restrict__ t,
-    const int* __restrict__ Nr, const int* __restrict__ Mr, int Npad, int Mpad, float k, float e,
-    float inv2k, float Kc, float aKc, int need_grad, float* V, float* dQ, float* dT) {
+    const int* __restrict__ Nr, const int* __restrict__ Mr, int K, int Npad, int Mpad, float k,
+    float e, float inv2k, float Kc, float aKc, int need_grad, float* V, float* dQ, float* dT) {
+  constexpr int kThreads = 32 * WARPS;
   extern __shared__ __align__(16) float4 smem[];
   __shared__ float red[96];
-  const int row = blockIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const size_t row = blockIdx.x;
   const int N = Nr ? min(max(Nr[row], 0), Npad) : Npad;
   const int M = Mr ? min(max(Mr[row], 0), Mpad) : Mpad;
-  float4* sP = smem;  // 2 * Npad (duplicated expanded reference)
+  float4* sP = smem;
   float4* sB = sP + 2 * Npad;
-  float2* sQc = reinterpret_cast<float2*>(sB + Mpad);
-  const float* a = A + (size_t)row * Npad * 3;
-  const float* b = B + (size_t)row * Mpad * 3;
-  // centroid of the real reference points
+  float2* sQ = reinterpret_cast<float2*>(sB + Mpad);
+  const float* a = A + row * Npad * 3;
+  const float* b = B + row * Mpad * 3;
+  for (int j = tid; j < M; j += kThreads)
+    sB[j] = make_float4(b[3 * j], b[3 * j + 1], b[3 * j + 2], ESP ? CB[row * Mpad + j] : 0.f);
   float3 s = make_float3(0.f, 0.f, 0.f);
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+  for (int i = tid; i < N; i += kThreads) {
     s.x += a[3 * i]; s.y += a[3 * i + 1]; s.z += a[3 * i + 2];
   }
   s = block_sum3(s, red);
   const float inv = 1.f / (float)(N > 0 ? N : 1);
   const float3 c = make_float3(s.x * inv, s.y * inv, s.z * inv);
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    const float ax = a[3 * i] - c.x, ay = a[3 * i + 1] - c.y, az = a[3 * i + 2] - c.z;
-    float w = -k * (ax * ax + ay * ay + az * az);
-    if (ESP) {
-      const float ci = CA[(size_t)row * Npad + i];
-      w = fmaf(-e * ci, ci, w);
-      sQc[i] = make_float2(2.f * e * ci, 2.f * e * ci);
-    }
-    const float px = 2.f * k * ax, py = 2.f * k * ay, pz = 2.f * k * az;
-    sP[2 * i] = make_float4(px, px, py, py);
-    sP[2 * i + 1] = make_float4(pz, pz, w, w);
-  }
-  for (int j = threadIdx.x; j < M; j += blockDim.x)
-    sB[j] = make_float4(b[3 * j], b[3 * j + 1], b[3 * j + 2],
-                        ESP ? CB[(size_t)row * Mpad + j] : 0.f);
+  for (int i = tid; i < N; i += kThreads)
+    expand_point<ESP>(a[3 * i] - c.x, a[3 * i + 1] - c.y, a[3 * i + 2] - c.z,
+                      ESP ? CA[row * Npad + i] : 0.f, k, e, sP + 2 * i, sQ + i);
   __syncthreads();
   float qq[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) qq[i] = q[(size_t)row * 4 + i];
+  for (int i = 0; i < 4; ++i) qq[i] = q[row * 4 + i];
   const Rot R = quat_to_rot(qq);
   Moments acc;
   acc.zero();
-  shape_pose<32, ESP>(sP, sQc, sB, N, M, threadIdx.x, R, t[(size_t)row * 3] - c.x,
-                      t[(size_t)row * 3 + 1] - c.y, t[(size_t)row * 3 + 2] - c.z, k, e, inv2k,
-                      acc);
-  acc.group_sum<32>();
-  acc.scale(Kc, aKc);
-  if (threadIdx.x == 0) {
-    V[row] = acc.v;
-    if (need_grad) {
-      float d[4];
-      quat_grad_from_moment(qq, acc.g, d);
+  shape_pose<kThreads, ESP, 2, 4>(sP, sQ, sB, N, M, tid, R, t[row * 3] - c.x, t[row * 3 + 1] - c.y,
+                                  t[row * 3 + 2] - c.z, k, e, inv2k, acc);
+  Reduced r;
+  r.from(acc, qq);
+  float own[1];
+  LanePose<32>::reduce(r, lane, own);
+  const int id = LanePose<32>::comp(lane, 0);
+  const float f = id == 0 ? Kc : aKc;
+  if (WARPS == 1) {
+    if (lane % 4 == 0) eval_write(id, own[0] * f, row, need_grad, V, dQ, dT);
+    return;
+  }
+  // red was last read before the barrier above
+  if (lane % 4 == 0) red[warp * 8 + id] = own[0];
+  __syncthreads();
+  if (tid < 8) {
+    float x = 0.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dQ[(size_t)row * 4 + i] = d[i];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) dT[(size_t)row * 3 + i] = acc.f[i];
-    }
+    for (int w = 0; w < WARPS; ++w) x += red[w * 8 + tid];
+    eval_write(tid, x * (tid == 0 ? Kc : aKc), row, need_grad, V, dQ, dT);
   }
 }
 
+// LANES lanes a pose, 32 / LANES poses to a warp: a few features leave most of a warp idle.  Fit
+// features visit the reference features of their own type only.  Bound by the latency around short
+// loops.  One B200, before (a warp a pose, every reference feature looked at) -> after: 13 000
+// poses of 3-20 features 20.9 -> 14.7 us (8 lanes), of 3-70 features 71.1 -> 41.4 (32 lanes).
+template <int LANES>
 __global__ void __launch_bounds__(32) pharm_eval_kernel(
     const float* __restrict__ A, const float* __restrict__ B, const float* __restrict__ RV,
     const float* __restrict__ FV, const int* __restrict__ At, const int* __restrict__ Bt,
     const float* __restrict__ q, const float* __restrict__ t, const int* __restrict__ Nr,
-    const int* __restrict__ Mr, int Npad, int Mpad, PharmTables tab, int need_grad, float* O,
-    float* dQ, float* dT) {
+    const int* __restrict__ Mr, int K, int Npad, int Mpad, int words, PharmTables tab,
+    int need_grad, float* O, float* dQ, float* dT) {
   extern __shared__ __align__(16) float4 smem[];
-  const int row = blockIdx.x;
+  constexpr int kPoses = 32 / LANES;   // poses of a warp
+  const int lane = threadIdx.x % LANES, grp = threadIdx.x / LANES;
+  const size_t first = (size_t)blockIdx.x * kPoses;
+  const bool active = first + grp < (size_t)K;   // groups past the last pose shadow it
+  const size_t row = active ? first + grp : (size_t)K - 1;
   const int N = Nr ? min(max(Nr[row], 0), Npad) : Npad;
   const int M = Mr ? min(max(Mr[row], 0), Mpad) : Mpad;
-  float4* sRA = smem;
+  float4* sRA = smem + 2 * ((size_t)Npad + Mpad) * grp;
   float4* sRV = sRA + Npad;
   float4* sFA = sRV + Npad;
   float4* sFV = sFA + Mpad;
-  const float* a = A + (size_t)row * Npad * 3;
-  const float* b = B + (size_t)row * Mpad * 3;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    int ty = At[(size_t)row * Npad + i];
-    ty = (ty < 0 || ty > 8) ? 8 : ty;  // out-of-table types are treated as Dummy
-    sRA[i] = make_float4(a[3 * i], a[3 * i + 1], a[3 * i + 2], __int_as_float(ty));
-    sRV[i] = RV ? unit4(RV[((size_t)row * Npad + i) * 3], RV[((size_t)row * Npad + i) * 3 + 1],
-                        RV[((size_t)row * Npad + i) * 3 + 2])
-                : make_float4(0.f, 0.f, 0.f, 0.f);
+  // Reference features grouped by type, in their order: bit i of sM[type] marks feature i, so a
+  // feature's place is the marks of earlier types and those below its own.  words = 0: left as
+  // they are (no room for the marks).
+  unsigned* sM = reinterpret_cast<unsigned*>(smem + 2 * ((size_t)Npad + Mpad) * kPoses) +
+                 (9 * words + 10) * grp;
+  int* off = reinterpret_cast<int*>(sM + 9 * words);
+  auto type_of = [](const int* ty, size_t i) {
+    const int u = ty[i];
+    return (u < 0 || u > 8) ? 8 : u;  // out-of-table types are treated as Dummy
+  };
+  if (words) {
+    for (int i = lane; i < 9 * words; i += LANES) sM[i] = 0;
+    __syncwarp();
+    for (int i = lane; i < N; i += LANES)
+      atomicOr(&sM[type_of(At, row * Npad + i) * words + i / 32], 1u << (i % 32));
+    __syncwarp();
+    for (int y = lane; y < 10; y += LANES) {
+      int n = 0;
+      for (int w = 0; w < y * words; ++w) n += __popc(sM[w]);
+      off[y] = n;
+    }
+    __syncwarp();
   }
-  for (int j = threadIdx.x; j < M; j += blockDim.x) {
-    int ty = Bt[(size_t)row * Mpad + j];
-    ty = (ty < 0 || ty > 8) ? 8 : ty;
-    sFA[j] = make_float4(b[3 * j], b[3 * j + 1], b[3 * j + 2], __int_as_float(ty));
-    sFV[j] = FV ? unit4(FV[((size_t)row * Mpad + j) * 3], FV[((size_t)row * Mpad + j) * 3 + 1],
-                        FV[((size_t)row * Mpad + j) * 3 + 2])
-                : make_float4(0.f, 0.f, 0.f, 0.f);
+  auto put = [&](const float* x, const float* v, int u, float4* a, float4* d) {
+    *a = make_float4(x[0], x[1], x[2], __int_as_float(u));
+    *d = v ? unit4(v[0], v[1], v[2]) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  for (int i = lane; i < N; i += LANES) {
+    const size_t g = row * Npad + i;
+    const int u = type_of(At, g);
+    int at = i;
+    if (words) {
+      const unsigned* m = sM + u * words;
+      at = off[u] + __popc(m[i / 32] & ((1u << (i % 32)) - 1));
+      for (int w = 0; w < i / 32; ++w) at += __popc(m[w]);
+    }
+    put(A + 3 * g, RV ? RV + 3 * g : nullptr, u, sRA + at, sRV + at);
   }
-  __syncthreads();
+  for (int j = lane; j < M; j += LANES) {
+    const size_t g = row * Mpad + j;
+    put(B + 3 * g, FV ? FV + 3 * g : nullptr, type_of(Bt, g), sFA + j, sFV + j);
+  }
+  __syncwarp();
   float qq[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) qq[i] = q[(size_t)row * 4 + i];
+  for (int i = 0; i < 4; ++i) qq[i] = q[row * 4 + i];
   const Rot R = quat_to_rot(qq);
   Moments acc;
   acc.zero();
-  pharm_pose<32>(sRA, sRV, sFA, sFV, N, M, threadIdx.x, R, t[(size_t)row * 3],
-                 t[(size_t)row * 3 + 1], t[(size_t)row * 3 + 2], tab, acc);
-  acc.group_sum<32>();
-  if (threadIdx.x == 0) {
-    O[row] = acc.v;
-    if (need_grad) {
-      float d[4];
-      quat_grad_from_moment(qq, acc.g, d);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) dQ[(size_t)row * 4 + i] = d[i];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) dT[(size_t)row * 3 + i] = acc.f[i];
-    }
-  }
+  pharm_pose<LANES>(sRA, sRV, sFA, sFV, N, M, lane, R, t[row * 3], t[row * 3 + 1],
+                    t[row * 3 + 2], tab, acc, words ? off : nullptr);
+  __syncwarp();
+  Reduced r;
+  r.from(acc, qq);
+  float own[1];
+  LanePose<LANES>::reduce(r, lane, own);
+  if (active && lane % (LANES / 8) == 0)
+    eval_write(LanePose<LANES>::comp(lane, 0), own[0], row, need_grad, O, dQ, dT);
 }
 
 __global__ void tanimoto_adam_kernel(const float* __restrict__ V, const float* __restrict__ dQ,
@@ -188,22 +246,19 @@ int overlap_eval_launch(const float* A, const float* B, const float* CA, const f
   const float e = esp ? (float)((double)inv_lam * 1.4426950408889634) : 0.f;
   const float inv2k = (float)(1.0 / (a * 1.4426950408889634));
   const double Kd = std::pow(M_PI, 1.5) / std::pow(2.0 * a, 1.5);
-  const size_t smem = sizeof(float4) * (2 * (size_t)Npad + Mpad) + sizeof(float2) * (size_t)Npad + 16;
-  cudaError_t ce;
-  if (esp) {
-    ce = cudaFuncSetAttribute(overlap_eval_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (ce == cudaSuccess)
-      overlap_eval_kernel<true><<<K, 32, smem, st>>>(A, B, CA, CB, q, t, Nr, Mr, Npad, Mpad, k, e,
-                                                     inv2k, (float)Kd, (float)(a * Kd), need_grad, V, dQ, dT);
-  } else {
-    ce = cudaFuncSetAttribute(overlap_eval_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (ce == cudaSuccess)
-      overlap_eval_kernel<false><<<K, 32, smem, st>>>(A, B, nullptr, nullptr, q, t, Nr, Mr, Npad,
-                                                      Mpad, k, 0.f, inv2k, (float)Kd, (float)(a * Kd),
-                                                      need_grad, V, dQ, dT);
-  }
+  const size_t smem = sizeof(float4) * (2 * (size_t)Npad + Mpad + (esp ? (Npad + 1) / 2 : 0));
+  // Above 64 fit points each lane of two warps has a whole register tile: 1600 poses of 60-100
+  // charged points 12.7 us with one warp and 12.5 with two, of 200-400 points 129 and 87.  Below,
+  // lanes of the second warp would have no point.
+  const bool wide = Mpad > 64;
+  const auto kern = esp ? (wide ? overlap_eval_kernel<true, 2> : overlap_eval_kernel<true, 1>)
+                        : (wide ? overlap_eval_kernel<false, 2> : overlap_eval_kernel<false, 1>);
+  const cudaError_t ce =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ce != cudaSuccess)
     return set_error(FSS_ERR_CUDA, std::string("fss_overlap_grad: ") + cudaGetErrorString(ce));
+  kern<<<K, wide ? 64 : 32, smem, st>>>(A, B, CA, CB, q, t, Nr, Mr, K, Npad, Mpad, k, e, inv2k,
+                                        (float)Kd, (float)(a * Kd), need_grad, V, dQ, dT);
   return check_launch("fss_overlap_grad");
 }
 
@@ -220,14 +275,35 @@ int pharm_eval_launch(const float* A, const float* B, const float* RV, const flo
     return set_error(FSS_ERR_INVALID, "fss_pharm_grad: directional scoring needs vectors");
   if (Npad > kMaxPoints || Mpad > kMaxPoints)
     return set_error(FSS_ERR_UNSUPPORTED, "fss_pharm_grad: more than fss_max_points() features");
-  const size_t smem = sizeof(float4) * 2 * ((size_t)Npad + Mpad) + 16;
-  cudaError_t ce = cudaFuncSetAttribute(pharm_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int dev = 0, optin = 0, sms = 0;
+  cudaError_t ce = cudaGetDevice(&dev);
+  if (ce == cudaSuccess)
+    ce = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (ce != cudaSuccess)
     return set_error(FSS_ERR_CUDA, std::string("fss_pharm_grad: ") + cudaGetErrorString(ce));
-  pharm_eval_kernel<<<K, 32, smem, st>>>(A, B, directional ? RV : nullptr,
-                                         directional ? FV : nullptr, At, Bt, q, t, Nr, Mr, Npad,
-                                         Mpad, make_pharm_tables(directional != 0), need_grad, O,
-                                         dQ, dT);
+  // the largest feature lists leave no room to group them by type
+  int words = (Npad + 31) / 32;
+  auto bytes = [&] {
+    return sizeof(float4) * 2 * ((size_t)Npad + Mpad) +
+           (words ? sizeof(int) * (9 * (size_t)words + 10) : 0);
+  };
+  if (bytes() > (size_t)optin) words = 0;
+  const size_t stage = bytes();
+  // Eight lanes a pose up to four fit features per lane and from one full wave of one-warp CTAs
+  // on; in us with 8 and with 32 lanes: 13 000 poses of 3-20 features 14.7 and 22.3, 3-30 19.9 and
+  // 23.2, 3-45 42.9 and 31.0; 100 poses of 3-20 10.4 and 5.5.
+  constexpr int kPoses = 32 / kFewLanes;
+  const bool small = Npad <= 32 && Mpad <= 32 && K > 32 * sms;
+  const int per_cta = small ? kPoses : 1;
+  const size_t smem = per_cta * stage;
+  const auto kern = small ? pharm_eval_kernel<kFewLanes> : pharm_eval_kernel<32>;
+  ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (ce != cudaSuccess)
+    return set_error(FSS_ERR_CUDA, std::string("fss_pharm_grad: ") + cudaGetErrorString(ce));
+  kern<<<(K - 1) / per_cta + 1, 32, smem, st>>>(
+      A, B, directional ? RV : nullptr, directional ? FV : nullptr, At, Bt, q, t, Nr, Mr, K, Npad,
+      Mpad, words, make_pharm_tables(directional != 0), need_grad, O, dQ, dT);
   return check_launch("fss_pharm_grad");
 }
 

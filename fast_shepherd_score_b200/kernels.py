@@ -30,13 +30,23 @@ _f32, _i32 = torch.float32, torch.int32
 
 
 def _c(t, dtype):
-    return t.to(dtype).contiguous()
+    return t if t.dtype is dtype and t.is_contiguous() else t.to(dtype).contiguous()
 
 
-def _counts(x, K, pad, device):
+def _counts(x, device):
+    """Real counts on the device, or None (every point real; the kernels take NULL for it)."""
     if x is None:
-        return torch.full((K,), pad, dtype=_i32, device=device)
+        return None
+    if isinstance(x, torch.Tensor) and x.device == device:
+        return _c(x, _i32)
     return torch.as_tensor(x, device=device).to(_i32).contiguous()
+
+
+def _pose_outputs(K, dev, need_grad):
+    """V (K,), dQ (K,4), dT (K,3); the kernels write every row of what they compute."""
+    new = torch.empty if need_grad else torch.zeros
+    return (torch.empty(K, dtype=_f32, device=dev), new(K, 4, dtype=_f32, device=dev),
+            new(K, 3, dtype=_f32, device=dev))
 
 
 def overlap_score_grad_se3_batch(A, B, q, t, *, alpha: float = 0.81, N_real=None, M_real=None,
@@ -60,10 +70,8 @@ def _overlap(A, B, CA, CB, q, t, alpha, inv_lam, N_real, M_real, need_grad):
     A, B, q, t = _c(A, _f32), _c(B, _f32), _c(q, _f32), _c(t, _f32)
     CA = None if CA is None else _c(CA, _f32)
     CB = None if CB is None else _c(CB, _f32)
-    Nr, Mr = _counts(N_real, K, N_pad, dev), _counts(M_real, K, M_pad, dev)
-    V = torch.empty(K, dtype=_f32, device=dev)
-    dQ = torch.zeros(K, 4, dtype=_f32, device=dev)
-    dT = torch.zeros(K, 3, dtype=_f32, device=dev)
+    Nr, Mr = _counts(N_real, dev), _counts(M_real, dev)
+    V, dQ, dT = _pose_outputs(K, dev, need_grad)
     L = _lib.load()
     check(L.fss_overlap_grad(ptr(A, _f32, "A"), ptr(B, _f32, "B"), ptr(CA, _f32, "charges_A"),
                              ptr(CB, _f32, "charges_B"), ptr(q, _f32, "q"), ptr(t, _f32, "t"),
@@ -101,10 +109,8 @@ def _pharm(A, B, RV, FV, At, Bt, q, t, N_real, M_real, directional, need_grad):
     RV = None if RV is None else _c(RV, _f32)
     FV = None if FV is None else _c(FV, _f32)
     At, Bt = _c(At, _i32), _c(Bt, _i32)
-    Nr, Mr = _counts(N_real, K, N_pad, dev), _counts(M_real, K, M_pad, dev)
-    O = torch.empty(K, dtype=_f32, device=dev)
-    dQ = torch.zeros(K, 4, dtype=_f32, device=dev)
-    dT = torch.zeros(K, 3, dtype=_f32, device=dev)
+    Nr, Mr = _counts(N_real, dev), _counts(M_real, dev)
+    O, dQ, dT = _pose_outputs(K, dev, need_grad)
     L = _lib.load()
     check(L.fss_pharm_grad(ptr(A, _f32), ptr(B, _f32), ptr(RV, _f32), ptr(FV, _f32),
                            ptr(At, _i32), ptr(Bt, _i32), ptr(q, _f32), ptr(t, _f32),
