@@ -33,43 +33,67 @@ LAM_SCALING = (1e4 / (4 * 55.263 * math.pi)) ** 2
 _f32, _i32 = torch.float32, torch.int32
 
 
+# Largest unit-gradient array (bytes) that a packed forward leaves for its backward.
+UNIT_BYTES = 256 << 20
+SMALL_POINTS = 64
+
+
 class PackedTanimoto(torch.autograd.Function):
-    """score_p = V_AB / (V_AA + V_BB - V_AB) for P pairs of packed clouds."""
+    """score_p = V_AB / (V_AA + V_BB - V_AB) for P pairs of packed clouds.
+
+    With ``grad_on`` and only the fit side differentiated, the forward of small clouds also
+    writes each pair's d score / d fit point (``fss_score_fwd_unit``) and the backward scales and
+    adds them; otherwise the backward evaluates the Gaussians again (``fss_score_bwd``)."""
 
     @staticmethod
     def forward(ctx, ref_pts, fit_pts, ref_off, fit_off, pair_ref, pair_fit, max_ref, max_fit,
-                alpha, esp, inv_lam):
+                alpha, esp, inv_lam, grad_on=False):
         dev = ref_pts.device
         P = int(pair_ref.shape[0])
         ref_pts, fit_pts = ref_pts.contiguous(), fit_pts.contiguous()
         score = torch.empty(P, dtype=_f32, device=dev)
         ov = torch.empty(P, 3, dtype=_f32, device=dev)
-        check(_lib.load().fss_score_fwd(ptr(ref_pts, _f32), ptr(ref_off, _i32), ptr(fit_pts, _f32),
-                                        ptr(fit_off, _i32), ptr(pair_ref, _i32),
-                                        ptr(pair_fit, _i32), P, int(max_ref), int(max_fit),
-                                        float(alpha), int(esp), float(inv_lam), ptr(score),
-                                        ptr(ov), stream_ptr(dev)), "score_fwd")
-        ctx.save_for_backward(ref_pts, fit_pts, ref_off, fit_off, pair_ref, pair_fit, ov)
+        need = ctx.needs_input_grad
+        unit = None
+        if (grad_on and need[1] and not need[0] and 0 < max_fit <= SMALL_POINTS
+                and max_ref <= SMALL_POINTS and 16 * P * int(max_fit) <= UNIT_BYTES):
+            unit = torch.empty(P, int(max_fit), 4, dtype=_f32, device=dev)
+        args = (ptr(ref_pts, _f32), ptr(ref_off, _i32), ptr(fit_pts, _f32), ptr(fit_off, _i32),
+                ptr(pair_ref, _i32), ptr(pair_fit, _i32), P, int(max_ref), int(max_fit),
+                float(alpha), int(esp), float(inv_lam), ptr(score), ptr(ov))
+        lib = _lib.load()
+        if unit is None:
+            check(lib.fss_score_fwd(*args, stream_ptr(dev)), "score_fwd")
+        else:
+            check(lib.fss_score_fwd_unit(*args, ptr(unit), stream_ptr(dev)), "score_fwd_unit")
+        ctx.save_for_backward(ref_pts, fit_pts, ref_off, fit_off, pair_ref, pair_fit, ov, unit)
         ctx.cfg = (int(max_ref), int(max_fit), float(alpha), int(esp), float(inv_lam))
         ctx.mark_non_differentiable(ov)
         return score, ov
 
     @staticmethod
     def backward(ctx, g_score, g_ov):
-        ref_pts, fit_pts, ref_off, fit_off, pair_ref, pair_fit, ov = ctx.saved_tensors
+        ref_pts, fit_pts, ref_off, fit_off, pair_ref, pair_fit, ov, unit = ctx.saved_tensors
         max_ref, max_fit, alpha, esp, inv_lam = ctx.cfg
         need_r, need_f = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         if not (need_r or need_f):
-            return (None,) * 11
+            return (None,) * 12
         gr = torch.zeros_like(ref_pts) if need_r else None
         gf = torch.zeros_like(fit_pts) if need_f else None
         g = g_score.to(_f32).contiguous()
-        check(_lib.load().fss_score_bwd(ptr(ref_pts, _f32), ptr(ref_off, _i32), ptr(fit_pts, _f32),
-                                        ptr(fit_off, _i32), ptr(pair_ref, _i32),
-                                        ptr(pair_fit, _i32), int(pair_ref.shape[0]), max_ref,
-                                        max_fit, alpha, esp, inv_lam, ptr(ov), ptr(g), ptr(gr),
-                                        ptr(gf), stream_ptr(ref_pts.device)), "score_bwd")
-        return gr, gf, None, None, None, None, None, None, None, None, None
+        P = int(pair_ref.shape[0])
+        lib, st = _lib.load(), stream_ptr(ref_pts.device)
+        if unit is not None:
+            check(lib.fss_score_bwd_unit(ptr(ref_off, _i32), ptr(fit_off, _i32),
+                                         ptr(pair_ref, _i32), ptr(pair_fit, _i32), P, max_ref,
+                                         max_fit, ptr(g), ptr(unit), ptr(gf), st),
+                  "score_bwd_unit")
+        else:
+            check(lib.fss_score_bwd(ptr(ref_pts, _f32), ptr(ref_off, _i32), ptr(fit_pts, _f32),
+                                    ptr(fit_off, _i32), ptr(pair_ref, _i32), ptr(pair_fit, _i32),
+                                    P, max_ref, max_fit, alpha, esp, inv_lam, ptr(ov), ptr(g),
+                                    ptr(gr), ptr(gf), st), "score_bwd")
+        return (gr, gf) + (None,) * 10
 
 
 def tanimoto_packed(ref_pts, ref_off, fit_pts, fit_off, pair_ref, pair_fit, *, alpha=0.81,
@@ -89,7 +113,8 @@ def tanimoto_packed(ref_pts, ref_off, fit_pts, fit_off, pair_ref, pair_fit, *, a
                                      fit_off.to(_i32).contiguous(),
                                      pair_ref.to(_i32).contiguous(), pair_fit.to(_i32).contiguous(),
                                      max_ref, max_fit, alpha, esp,
-                                     1.0 / float(lam) if esp else 0.0)
+                                     1.0 / float(lam) if esp else 0.0,
+                                     torch.is_grad_enabled())
     return (score, ov) if return_overlaps else score
 
 

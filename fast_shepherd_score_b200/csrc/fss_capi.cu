@@ -57,7 +57,11 @@ int seeds_launch(const float* ref_pts, const int32_t* ref_off, const float* fit_
 int score_fwd_launch(const float* ref_pts, const int32_t* ref_off, const float* fit_pts,
                      const int32_t* fit_off, const int32_t* pair_ref, const int32_t* pair_fit,
                      int P, int maxN, int maxM, float alpha, int esp, float inv_lam, float* score,
-                     float* overlaps, cudaStream_t st);
+                     float* overlaps, float* unit_fit, cudaStream_t st);
+int score_bwd_unit_launch(const int32_t* ref_off, const int32_t* fit_off, const int32_t* pair_ref,
+                          const int32_t* pair_fit, int P, int maxN, int maxM,
+                          const float* grad_score, const float* unit_fit, float* grad_fit,
+                          cudaStream_t st);
 int score_bwd_launch(const float* ref_pts, const int32_t* ref_off, const float* fit_pts,
                      const int32_t* fit_off, const int32_t* pair_ref, const int32_t* pair_fit,
                      int P, int maxN, int maxM, float alpha, int esp, float inv_lam,
@@ -187,7 +191,28 @@ int fss_score_fwd(const float* ref_pts, const int32_t* ref_off, const float* fit
                   int32_t esp, float inv_lam, float* score, float* overlaps, void* stream) {
   FSS_GUARD(fss::score_fwd_launch(ref_pts, ref_off, fit_pts, fit_off, pair_ref, pair_fit,
                                   n_pairs, max_ref_points, max_fit_points, alpha, esp, inv_lam,
-                                  score, overlaps, S(stream)));
+                                  score, overlaps, nullptr, S(stream)));
+}
+
+int fss_score_fwd_unit(const float* ref_pts, const int32_t* ref_off, const float* fit_pts,
+                       const int32_t* fit_off, const int32_t* pair_ref, const int32_t* pair_fit,
+                       int32_t n_pairs, int32_t max_ref_points, int32_t max_fit_points,
+                       float alpha, int32_t esp, float inv_lam, float* score, float* overlaps,
+                       float* unit_fit, void* stream) {
+  if (!unit_fit && n_pairs > 0)
+    return fss::set_error(FSS_ERR_INVALID, "fss_score_fwd_unit: null pointer");
+  FSS_GUARD(fss::score_fwd_launch(ref_pts, ref_off, fit_pts, fit_off, pair_ref, pair_fit,
+                                  n_pairs, max_ref_points, max_fit_points, alpha, esp, inv_lam,
+                                  score, overlaps, unit_fit, S(stream)));
+}
+
+int fss_score_bwd_unit(const int32_t* ref_off, const int32_t* fit_off, const int32_t* pair_ref,
+                       const int32_t* pair_fit, int32_t n_pairs, int32_t max_ref_points,
+                       int32_t max_fit_points, const float* grad_score, const float* unit_fit,
+                       float* grad_fit, void* stream) {
+  FSS_GUARD(fss::score_bwd_unit_launch(ref_off, fit_off, pair_ref, pair_fit, n_pairs,
+                                       max_ref_points, max_fit_points, grad_score, unit_fit,
+                                       grad_fit, S(stream)));
 }
 
 int fss_score_bwd(const float* ref_pts, const int32_t* ref_off, const float* fit_pts,

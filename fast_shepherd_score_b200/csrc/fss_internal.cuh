@@ -14,6 +14,7 @@ namespace fss {
 // Hard limit of points (or pharmacophore features) per molecule that the fused kernels
 // stage in shared memory.  4096 float4 points = 64 KB per cloud.
 constexpr int kMaxPoints = 4096;
+constexpr int kSmallPoints = 64;   // clouds that fss_score_small.cu scores
 
 // Thread-local error message + status helpers (fss_capi.cu).
 int set_error(int code, const std::string& msg);
@@ -181,6 +182,13 @@ __device__ __forceinline__ void stage_fit_pharm(const Pts ga, const Pts gv, int 
 PharmTables make_pharm_tables(bool directional);
 
 int num_sms();
+
+// fss_score_small.cu: packed scores of clouds of at most kSmallPoints points; unit_fit may be null
+int score_small_launch(const float* ref_pts, const int32_t* ref_off, const float* fit_pts,
+                       const int32_t* fit_off, const int32_t* pair_ref, const int32_t* pair_fit,
+                       int P, int maxN, int maxM, float nk, float ne, float Kc, float aKc,
+                       float cKc, int esp, float* score, float* overlaps, float* unit_fit,
+                       cudaStream_t st);
 
 // Launchers behind the C ABI (each validates its arguments and returns an fss_status).
 int align_launch(const fss_align_desc* d, cudaStream_t st);

@@ -260,6 +260,22 @@ int fss_score_bwd(const float *ref_pts, const int32_t *ref_off, const float *fit
                   int32_t esp, float inv_lam, const float *overlaps, const float *grad_score,
                   float *grad_ref, float *grad_fit, void *stream);
 
+/* fss_score_fwd, and in the same pass d(score_p)/d(point k of its fit molecule) in
+ * unit_fit[4 (p max_fit_points + k) + 0..3] (x, y, z, charge; 0 without esp), for clouds of at
+ * most 64 points: FSS_ERR_UNSUPPORTED, with nothing written, when a max_*_points is larger.
+ * Scores and overlaps are those of fss_score_fwd bit for bit.  fss_score_bwd_unit ADDS
+ * grad_score[p] times those rows into grad_fit, what fss_score_bwd adds up to the order of its
+ * roundings. */
+int fss_score_fwd_unit(const float *ref_pts, const int32_t *ref_off, const float *fit_pts,
+                       const int32_t *fit_off, const int32_t *pair_ref, const int32_t *pair_fit,
+                       int32_t n_pairs, int32_t max_ref_points, int32_t max_fit_points,
+                       float alpha, int32_t esp, float inv_lam, float *score, float *overlaps,
+                       float *unit_fit, void *stream);
+int fss_score_bwd_unit(const int32_t *ref_off, const int32_t *fit_off, const int32_t *pair_ref,
+                       const int32_t *pair_fit, int32_t n_pairs, int32_t max_ref_points,
+                       int32_t max_fit_points, const float *grad_score, const float *unit_fit,
+                       float *grad_fit, void *stream);
+
 /* Dense-batch form of fss_score_fwd / fss_score_bwd for the reference's padded tensors: ref
  * molecule b is ref_xyz[b, 0:ref_points, :] of a (B_ref, ref_points, 3) array (every point
  * real) with charges ref_q[b, :] (B_ref, ref_points) when esp != 0 (NULL otherwise); likewise
