@@ -29,6 +29,10 @@ SEED_BYTES = 16 + 12
 # per pair: index pair (8), cost order (4 + sort scratch 16), outputs (32), self overlaps (8)
 PAIR_BYTES = 8 + 20 + 32 + 8
 
+# calls that need no more run without asking for the free memory (an out-of-memory error halves
+# them as any other)
+SMALL_BYTES = 64 << 20
+
 _HOOK: Optional[Callable[[int, torch.device], int]] = None
 _LOCK = threading.Lock()
 LAST_CHUNKS: list = []   # chunk sizes of the most recent chunked call (for reports and tests)
@@ -94,7 +98,9 @@ def run_chunked(n: int, per_item_bytes: int, process: Callable[[int, int], Seque
     if n <= 0:
         return process(0, n)
     if budget is None:
-        budget = (budget_bytes(device, n * per_item_bytes) if torch.device(device).type == "cuda"
+        # asking the driver for the free memory costs 0.1 ms and more: a call this small tries
+        budget = (budget_bytes(device, n * per_item_bytes)
+                  if torch.device(device).type == "cuda" and n * per_item_bytes > SMALL_BYTES
                   else 1 << 62)
     chunk = max(1, min(n, int(budget // max(1, per_item_bytes))))
     if max_chunk:
