@@ -69,6 +69,10 @@ _SIGS = {
     "fss_pick_best": ([_vp] * 3 + [_i32, _i32] + [_vp] * 4, ctypes.c_int),
     "fss_score_fwd": ([_vp] * 6 + [_i32, _i32, _i32, _f32, _i32, _f32, _vp, _vp, _vp],
                       ctypes.c_int),
+    "fss_pair_cost": ([_vp] * 4 + [_i32] * 3 + [_vp] * 3, ctypes.c_int),
+    "fss_pad_anchors": ([_vp, _vp, _i32, _i32, _vp, _vp], ctypes.c_int),
+    "fss_centre_anchors": ([_vp, _vp, _i32] + [_vp] * 5, ctypes.c_int),
+    "fss_fold_centroids": ([_vp] * 6 + [_i32, _vp, _vp], ctypes.c_int),
     "fss_score_fwd_unit": ([_vp] * 6 + [_i32, _i32, _i32, _f32, _i32, _f32] + [_vp] * 4,
                            ctypes.c_int),
     "fss_score_bwd_unit": ([_vp] * 4 + [_i32] * 3 + [_vp] * 4, ctypes.c_int),

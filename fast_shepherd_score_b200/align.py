@@ -32,7 +32,7 @@ import torch
 
 from . import _lib, autotune, kernels, legacy_seeds, memory
 from ._lib import AlignDesc, check, ptr, stream_ptr
-from .layout import CloudSet, PharmSet, cost_order_device
+from .layout import CloudSet, PharmSet
 
 _f32, _i32 = torch.float32, torch.int32
 # Tversky weights of the reference (accel/drivers/pharm.py:40)
@@ -153,11 +153,11 @@ def align_packed(mode: str, *, pair_ref, pair_fit, seed_q, seed_t, steps: int, l
     n_fit = fit.n_mol if shape else fit_ph.n_mol
     if shape and pharm and (ref_ph.n_mol != n_ref or fit_ph.n_mol != n_fit):
         raise ValueError("shape and pharmacophore sets must describe the same molecules")
-    if P and validate:
-        # one device-to-host read for the four bounds
-        rmin, fmin, rmax, fmax = torch.stack([pair_ref.min(), pair_fit.min(), pair_ref.max(),
-                                              pair_fit.max()]).tolist()
-        if min(rmin, fmin) < 0 or rmax >= n_ref or fmax >= n_fit:
+    cost = None
+    if P and (validate or (order is None and P > 1)):
+        cr, cf = (ref, fit) if shape else (ref_ph, fit_ph)
+        cost, bad = kernels.pair_cost(cr.off, cf.off, pair_ref, pair_fit, n_ref, n_fit, validate)
+        if validate and bad.item():   # the call's one device-to-host read before the launch
             raise ValueError("pair index outside the molecule tables")
     if shape:
         esp_self = m == _lib.MODE_ESP
@@ -177,8 +177,7 @@ def align_packed(mode: str, *, pair_ref, pair_fit, seed_q, seed_t, steps: int, l
             if fit_self_ph is None:
                 fit_self_ph = kernels.pharm_self_overlap(fit_ph, directional)
     if order is None and P > 1:
-        cr, cf = (ref, fit) if shape else (ref_ph, fit_ph)
-        order = cost_order_device(cr.off, cf.off, pair_ref, pair_fit)
+        order = torch.argsort(cost, stable=True).to(_i32)
     tuned = (lanes_per_pose == 0 and chunks == 0 and cta_per_sm == 0 and accumulate == 0
              and kernel_variant == 0 and autotune.enabled() and P >= 64 and steps > 0)
     if tuned:

@@ -241,8 +241,8 @@ def _align_device_once(mode, ref: Optional[CloudSet], fit: Optional[CloudSet],
                   only_extended=only_extended, **tile)
         shift = None
         if mode == "pharm":
-            rph, shift = _centred_pharm(ref_ph)
-            g_ref, g_fit = _as_cloud(rph), _as_cloud(_centred_pharm(fit_ph)[0])
+            _, g_ref, shift = _centred_pharm(ref_ph)
+            g_fit = _centred_pharm(fit_ph)[1]
         elif mode in ESP_COMBO_MODES:
             g_ref, g_fit = tile["ref_surf"], tile["fit_surf"]
         else:
@@ -287,10 +287,10 @@ def _align_device_once(mode, ref: Optional[CloudSet], fit: Optional[CloudSet],
     if mode == "pharm":
         # the reference optimises each pair on per-cloud centred pharmacophores and folds
         # the centroids back into the translation (pharm.py:205-225, :509-517)
-        rph, c_ref = _centred_pharm(ref_ph)
-        fph, c_fit = _centred_pharm(fit_ph)
+        rph, r_cloud, c_ref = _centred_pharm(ref_ph)
+        fph, f_cloud, c_fit = _centred_pharm(fit_ph)
         if seeds is None:
-            seeds = K.seeds(_as_cloud(rph), _as_cloud(fph), pair_ref, pair_fit, num_seeds)
+            seeds = K.seeds(r_cloud, f_cloud, pair_ref, pair_fit, num_seeds)
         res = al.align_packed("pharm", ref_ph=rph, fit_ph=fph, pair_ref=pair_ref,
                               pair_fit=pair_fit, seed_q=seeds[0], seed_t=seeds[1],
                               steps=steps, lr=lr, ref_self=ref_self, fit_self=fit_self,
@@ -298,12 +298,8 @@ def _align_device_once(mode, ref: Optional[CloudSet], fit: Optional[CloudSet],
                               pharm_extended=al.extended_code(extended_points, only_extended),
                               **tile)
         sc, q, t = res
-        cr = c_ref[pair_ref.long()]
-        cf = c_fit[pair_fit.long()]
-        t = t - torch.einsum("bij,bj->bi", al._quat_rot(q), cf) + cr
-        rows = res.rows
-        out = al.AlignResult((sc, q, t))
-        out.rows = rows
+        out = al.AlignResult((sc, q, K.fold_centroids(q, t, pair_ref, pair_fit, c_ref, c_fit)))
+        out.rows = res.rows
         return out
     if seeds is None:
         seeds = K.seeds(ref, fit, pair_ref, pair_fit, num_seeds)
@@ -316,30 +312,10 @@ def _align_device_once(mode, ref: Optional[CloudSet], fit: Optional[CloudSet],
 
 
 def _centred_pharm(ps: PharmSet):
-    """The set with every molecule's anchors centred on its own centroid (types kept).  The
-    centroid is a padded per-molecule sum (the reference's masked sum, pharm.py:215-219), so
-    it is deterministic (an atomic scatter-add would make the last bits run-dependent)."""
+    """The set with every molecule's anchors centred on its own centroid (types kept), the centred
+    anchors as a plain cloud (for seeding), and the centroids."""
     if ps.anc.dtype != torch.float32:
         raise ValueError("mode 'pharm' re-centres its anchors: it needs float32 sets")
-    dev = ps.anc.device
-    n = torch.as_tensor(ps.counts, device=dev)
-    mol = torch.repeat_interleave(torch.arange(len(ps.counts), device=dev), n)
-    xyz = ps.anc[:, :3]
-    L = max(int(ps.max_points), 1)
-    ar = torch.arange(L, device=dev)[None, :]
-    off = torch.cumsum(n, 0) - n
-    mask = ar < n[:, None]
-    rows = torch.where(mask, off[:, None] + ar, torch.zeros_like(ar))
-    pts = xyz[rows] if xyz.shape[0] else torch.zeros(len(ps.counts), L, 3, device=dev)
-    c = torch.where(mask[..., None], pts, torch.zeros_like(pts)).sum(1)
-    c = c / n.clamp(min=1).to(xyz.dtype)[:, None]
-    anc = ps.anc.clone()
-    anc[:, :3] = xyz - c[mol]
-    return PharmSet(anc, ps.vec, ps.off, ps.counts, ps.max_points), c
-
-
-def _as_cloud(ps: PharmSet) -> CloudSet:
-    """Anchor positions of a pharmacophore set as a plain point cloud (for seeding)."""
-    pts = torch.zeros_like(ps.anc)
-    pts[:, :3] = ps.anc[:, :3]
-    return CloudSet(pts, ps.off, ps.counts, ps.max_points)
+    anc, pts, c = K.centre_anchors(ps)
+    return (PharmSet(anc, ps.vec, ps.off, ps.counts, ps.max_points),
+            CloudSet(pts, ps.off, ps.counts, ps.max_points), c)

@@ -54,6 +54,15 @@ int seeds_launch(const float* ref_pts, const int32_t* ref_off, const float* fit_
                  const int32_t* fit_off, const int32_t* pair_ref, const int32_t* pair_fit,
                  int P, int S, const float* fibo, int n_fibo, int fit_f16, float* sq, float* st,
                  cudaStream_t stream);
+int pair_cost_launch(const int32_t* roff, const int32_t* foff, const int32_t* pr,
+                     const int32_t* pf, int P, int n_ref, int n_fit, int32_t* key, int32_t* bad,
+                     cudaStream_t st);
+int pad_anchors_launch(const float* anc, const int32_t* off, int n_mol, int L, float* out,
+                       cudaStream_t st);
+int centre_anchors_launch(const float* anc, const int32_t* off, int n_mol, const float* sum,
+                          float* centred, float* cloud, float* centroid, cudaStream_t st);
+int fold_centroids_launch(const float* q, const float* t, const int32_t* pr, const int32_t* pf,
+                          const float* cr, const float* cf, int P, float* out, cudaStream_t st);
 int score_fwd_launch(const float* ref_pts, const int32_t* ref_off, const float* fit_pts,
                      const int32_t* fit_off, const int32_t* pair_ref, const int32_t* pair_fit,
                      int P, int maxN, int maxM, float alpha, int esp, float inv_lam, float* score,
@@ -183,6 +192,31 @@ int fss_pick_best(const float* row_score, const float* row_q, const float* row_t
                   float* out_t, void* stream) {
   FSS_GUARD(fss::pick_best_launch(row_score, row_q, row_t, n_pairs, n_starts, out_score, out_q,
                                   out_t, S(stream)));
+}
+
+int fss_pair_cost(const int32_t* ref_off, const int32_t* fit_off, const int32_t* pair_ref,
+                  const int32_t* pair_fit, int32_t n_pairs, int32_t n_ref, int32_t n_fit,
+                  int32_t* key, int32_t* bad, void* stream) {
+  FSS_GUARD(fss::pair_cost_launch(ref_off, fit_off, pair_ref, pair_fit, n_pairs, n_ref, n_fit, key,
+                                  bad, S(stream)));
+}
+
+int fss_pad_anchors(const float* anchors, const int32_t* off, int32_t n_mol, int32_t max_features,
+                    float* padded, void* stream) {
+  FSS_GUARD(fss::pad_anchors_launch(anchors, off, n_mol, max_features, padded, S(stream)));
+}
+
+int fss_centre_anchors(const float* anchors, const int32_t* off, int32_t n_mol, const float* sums,
+                       float* centred, float* cloud, float* centroids, void* stream) {
+  FSS_GUARD(fss::centre_anchors_launch(anchors, off, n_mol, sums, centred, cloud, centroids,
+                                       S(stream)));
+}
+
+int fss_fold_centroids(const float* q, const float* t, const int32_t* pair_ref,
+                       const int32_t* pair_fit, const float* ref_centroids,
+                       const float* fit_centroids, int32_t n_pairs, float* out, void* stream) {
+  FSS_GUARD(fss::fold_centroids_launch(q, t, pair_ref, pair_fit, ref_centroids, fit_centroids,
+                                       n_pairs, out, S(stream)));
 }
 
 int fss_score_fwd(const float* ref_pts, const int32_t* ref_off, const float* fit_pts,

@@ -166,6 +166,49 @@ def points(t: torch.Tensor, name: str = "points"):
     return ptr(t, _f32, name), 0
 
 
+def pair_cost(ref_off, fit_off, pair_ref, pair_fit, n_ref, n_fit, check_range=True):
+    """Sort keys of the pairs (minus the product of their sizes, int32) and, with ``check_range``, a
+    one-element tensor that is 1 when a pair lies outside the molecule tables (else None)."""
+    dev = pair_ref.device
+    P = int(pair_ref.shape[0])
+    key = torch.empty(P, dtype=_i32, device=dev)
+    bad = torch.zeros(1, dtype=_i32, device=dev) if check_range else None
+    check(_lib.load().fss_pair_cost(ptr(ref_off, _i32), ptr(fit_off, _i32), ptr(pair_ref, _i32),
+                                    ptr(pair_fit, _i32), P, int(n_ref), int(n_fit), ptr(key),
+                                    ptr(bad), stream_ptr(dev)), "pair_cost")
+    return key, bad
+
+
+def centre_anchors(ph):
+    """A pharmacophore set's anchors centred per molecule (types kept), the same positions as plain
+    points (w = 0), and the centroids (n_mol, 3).  The centroid is a padded per-molecule sum (the
+    reference's masked sum, pharm.py:215-219), so it is deterministic (an atomic scatter-add would
+    make the last bits run-dependent)."""
+    dev = ph.anc.device
+    n, L = ph.n_mol, max(int(ph.max_points), 1)
+    padded = torch.empty(n, L, 3, dtype=_f32, device=dev)
+    anc, off = ph.anc.contiguous(), ptr(ph.off, _i32)
+    lib, st = _lib.load(), stream_ptr(dev)
+    check(lib.fss_pad_anchors(ptr(anc, _f32), off, n, L, ptr(padded), st), "pad_anchors")
+    sums = padded.sum(1)
+    centred, cloud, c = torch.empty_like(anc), torch.empty_like(anc), torch.empty_like(sums)
+    check(lib.fss_centre_anchors(ptr(anc), off, n, ptr(sums), ptr(centred), ptr(cloud), ptr(c), st),
+          "centre_anchors")
+    return centred, cloud, c
+
+
+def fold_centroids(q, t, pair_ref, pair_fit, c_ref, c_fit):
+    """t - R(q) c_fit + c_ref per pair."""
+    P = int(q.shape[0])
+    pair_ref = _c(torch.as_tensor(pair_ref, device=q.device), _i32)
+    pair_fit = _c(torch.as_tensor(pair_fit, device=q.device), _i32)
+    out = torch.empty_like(t)
+    check(_lib.load().fss_fold_centroids(ptr(q, _f32), ptr(t, _f32), ptr(pair_ref), ptr(pair_fit),
+                                         ptr(c_ref), ptr(c_fit), P, ptr(out),
+                                         stream_ptr(q.device)), "fold_centroids")
+    return out
+
+
 def self_overlap(cs: CloudSet, alpha: float, esp: bool = False, lam: Optional[float] = None):
     """Per-molecule self overlap of a packed cloud set (shape, or ESP with lam)."""
     out = torch.empty(cs.n_mol, dtype=_f32, device=cs.device)

@@ -238,6 +238,25 @@ int fss_pick_best(const float *row_score, const float *row_q, const float *row_t
                   int32_t n_pairs, int32_t n_starts, float *out_score, float *out_q,
                   float *out_t, void *stream);
 
+/* Before and after an alignment.  fss_pair_cost: key[p] = -(points of the pair's reference x of its
+ * fit molecule) for an ascending stable sort into fss_align_desc.order; a pair outside the
+ * n_ref / n_fit molecules reads nothing, gets key 0 and sets *bad to 1 (bad may be NULL; zero it
+ * first).  fss_pad_anchors: the (n_mol, max_features, 3) padded anchors, 0 past a molecule's last.
+ * fss_centre_anchors: centroids (n_mol, 3) = sums / size (1 for an empty molecule), the anchors
+ * moved to them (types kept) and the same positions with w = 0.  fss_fold_centroids: out =
+ * t - R(q / |q|) fit_centroid + ref_centroid per pair (pharm.py:509-517). */
+int fss_pair_cost(const int32_t *ref_off, const int32_t *fit_off, const int32_t *pair_ref,
+                  const int32_t *pair_fit, int32_t n_pairs, int32_t n_ref, int32_t n_fit,
+                  int32_t *key, int32_t *bad, void *stream);
+int fss_pad_anchors(const float *anchors, const int32_t *off, int32_t n_mol,
+                    int32_t max_features, float *padded, void *stream);
+int fss_centre_anchors(const float *anchors, const int32_t *off, int32_t n_mol,
+                       const float *sums, float *centred, float *cloud, float *centroids,
+                       void *stream);
+int fss_fold_centroids(const float *q, const float *t, const int32_t *pair_ref,
+                       const int32_t *pair_fit, const float *ref_centroids,
+                       const float *fit_centroids, int32_t n_pairs, float *out, void *stream);
+
 /* ---------------------------------------------------------------------------------------
  * Differentiable scoring (coordinate / charge adjoint).
  * Replaces torch autograd through get_overlap / get_overlap_esp
