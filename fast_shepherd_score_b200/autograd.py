@@ -35,13 +35,13 @@ _f32, _i32 = torch.float32, torch.int32
 
 # Largest unit-gradient array (bytes) that a packed forward leaves for its backward.
 UNIT_BYTES = 256 << 20
-SMALL_POINTS = 64
+UNIT_POINTS = 512
 
 
 class PackedTanimoto(torch.autograd.Function):
     """score_p = V_AB / (V_AA + V_BB - V_AB) for P pairs of packed clouds.
 
-    With ``grad_on`` and only the fit side differentiated, the forward of small clouds also
+    With ``grad_on`` and only the fit side differentiated, the forward of clouds of up to 512 points also
     writes each pair's d score / d fit point (``fss_score_fwd_unit``) and the backward scales and
     adds them; otherwise the backward evaluates the Gaussians again (``fss_score_bwd``)."""
 
@@ -55,8 +55,8 @@ class PackedTanimoto(torch.autograd.Function):
         ov = torch.empty(P, 3, dtype=_f32, device=dev)
         need = ctx.needs_input_grad
         unit = None
-        if (grad_on and need[1] and not need[0] and 0 < max_fit <= SMALL_POINTS
-                and max_ref <= SMALL_POINTS and 16 * P * int(max_fit) <= UNIT_BYTES):
+        if (grad_on and need[1] and not need[0] and 0 < max_fit <= UNIT_POINTS
+                and max_ref <= UNIT_POINTS and 16 * P * int(max_fit) <= UNIT_BYTES):
             unit = torch.empty(P, int(max_fit), 4, dtype=_f32, device=dev)
         args = (ptr(ref_pts, _f32), ptr(ref_off, _i32), ptr(fit_pts, _f32), ptr(fit_off, _i32),
                 ptr(pair_ref, _i32), ptr(pair_fit, _i32), P, int(max_ref), int(max_fit),

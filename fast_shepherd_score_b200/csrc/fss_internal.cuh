@@ -14,7 +14,8 @@ namespace fss {
 // Hard limit of points (or pharmacophore features) per molecule that the fused kernels
 // stage in shared memory.  4096 float4 points = 64 KB per cloud.
 constexpr int kMaxPoints = 4096;
-constexpr int kSmallPoints = 64;   // clouds that fss_score_small.cu scores
+constexpr int kSmallPoints = 64;   // clouds that fss_score_small.cu scores with a warp a pair
+constexpr int kWidePoints = 512;   // and with a CTA a pair
 
 // Thread-local error message + status helpers (fss_capi.cu).
 int set_error(int code, const std::string& msg);

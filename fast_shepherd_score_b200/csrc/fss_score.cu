@@ -635,16 +635,17 @@ int score_fwd_launch(const float* ref_pts, const int32_t* ref_off, const float* 
   if (P == 0) return FSS_OK;
   if (!ref_pts || !ref_off || !fit_pts || !fit_off || !pair_ref || !pair_fit || !score || !overlaps)
     return set_error(FSS_ERR_INVALID, "fss_score_fwd: null pointer");
-  // a warp's registers hold a row of every 16th point: four rows a lane are what fits; larger
-  // clouds fill a CTA each (30 pairs of 15-60 points 5.3 us there and 5.7 here, 20 000 91 and 64)
-  if (maxN <= kSmallPoints && maxM <= kSmallPoints) {
+  // four rows a lane and eight warps a pair are what the registers hold; larger clouds take the
+  // thread-per-row kernels (which lose from 30 pairs of 15-60 points, 5.4 + 4.2 us against 6.0 + 1.9,
+  // to 1000 of 100-400, 161 + 165 against 186 + 4)
+  if (maxN <= kWidePoints && maxM <= kWidePoints) {
     const ScoreConsts c = score_consts(alpha, esp, inv_lam);
     return score_small_launch(ref_pts, ref_off, fit_pts, fit_off, pair_ref, pair_fit, P, maxN,
                               maxM, c.nk, c.ne, c.Kc, c.aKc, c.cKc, esp, score, overlaps, unit_fit,
                               st);
   }
   if (unit_fit)
-    return set_error(FSS_ERR_UNSUPPORTED, "fss_score_fwd_unit: clouds above 64 points");
+    return set_error(FSS_ERR_UNSUPPORTED, "fss_score_fwd_unit: clouds above 512 points");
   const PackedSrc R{reinterpret_cast<const float4*>(ref_pts), ref_off};
   const PackedSrc F{reinterpret_cast<const float4*>(fit_pts), fit_off};
   return fwd_dispatch(R, F, pair_ref, pair_fit, P, maxN, maxM, alpha, esp, inv_lam, score,

@@ -281,7 +281,7 @@ int fss_score_bwd(const float *ref_pts, const int32_t *ref_off, const float *fit
 
 /* fss_score_fwd, and in the same pass d(score_p)/d(point k of its fit molecule) in
  * unit_fit[4 (p max_fit_points + k) + 0..3] (x, y, z, charge; 0 without esp), for clouds of at
- * most 64 points: FSS_ERR_UNSUPPORTED, with nothing written, when a max_*_points is larger.
+ * most 512 points: FSS_ERR_UNSUPPORTED, with nothing written, when a max_*_points is larger.
  * Scores and overlaps are those of fss_score_fwd bit for bit.  fss_score_bwd_unit ADDS
  * grad_score[p] times those rows into grad_fit, what fss_score_bwd adds up to the order of its
  * roundings. */

@@ -1,4 +1,4 @@
-"""GPU parity of the packed scores of small clouds and their gradients with a float64 evaluation,
+"""GPU parity of the packed scores of clouds of up to 512 points and their gradients with a float64 evaluation,
 at the sizes where a cloud changes its rows per lane or its padding, with a shared reference, with
 changing ones and with molecules of several pairs.  Tolerances: scores 1e-5 (float32 sums of
 Gaussians), gradients 1e-4 relative to the largest component, as test_gpu_kernels has them."""
@@ -9,6 +9,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 SIZES = [1, 2, 3, 4, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64]
+WIDE = [65, 100, 127, 128, 129, 200, 256, 257, 400, 511, 512]
 
 
 def _set(rng, sizes, spread):
@@ -30,13 +31,13 @@ def _score64(x, y, lam):
 
 @pytest.mark.parametrize("lam", [None, 0.3])
 @pytest.mark.parametrize("shared", [True, False])
-@pytest.mark.parametrize("repeat", [1, 400])
-def test_small_scores_and_gradients(cuda, lam, shared, repeat):
+@pytest.mark.parametrize("sizes,repeat", [(SIZES, 1), (SIZES, 400), (WIDE + [1, 64], 1)])
+def test_small_scores_and_gradients(cuda, lam, shared, sizes, repeat):
     from fast_shepherd_score_b200 import autograd as ag
     rng = np.random.default_rng(5)
-    rp, ro = _set(rng, SIZES, 3.)
-    fp, fo = _set(rng, SIZES[::-1], 3.)
-    n = len(SIZES)
+    rp, ro = _set(rng, sizes, 3.)
+    fp, fo = _set(rng, sizes[::-1], 3.)
+    n = len(sizes)
     pf = np.tile(np.arange(n, dtype=np.int32), repeat)
     pr = np.full_like(pf, 9) if shared else ((pf * 4 + 1) % n).astype(np.int32)
     t = {k: torch.as_tensor(v, device=cuda) for k, v in
