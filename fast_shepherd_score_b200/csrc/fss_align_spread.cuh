@@ -244,26 +244,26 @@ __device__ __forceinline__ void add_point(Moments& acc, float inv2k, float4 b, f
                 __fmaf_rn(gz, inv2k, __fmul_rn(-z, g)), b.x, b.y, b.z);
 }
 
-// Up to four points per lane (j0 + u * stride) with the exponent factored or not, in scalar
-// arithmetic: the path of poses with a point beyond the factored exponent's range.
-template <bool ESP>
-__device__ __noinline__ void far_points(const ShapeArgs& a, const Rot& R, int j0, int stride,
-                                        int count, bool plain, Moments& acc) {
-  float4 b[4];
-  float x[4], y[4], z[4], w[4], sg[4], sx[4], sy[4], sz[4];
+// COUNT points per lane (j0 + u * LPP) with the unfactored exponent.
+template <int LPP, bool ESP, int COUNT, int UNR>
+__device__ __forceinline__ void far_points(const ShapeArgs& a, const Rot& R, int j0,
+                                           Moments& acc) {
+  float4 b[COUNT];
+  float x[COUNT], y[COUNT], z[COUNT], w[COUNT], sg[COUNT], sx[COUNT], sy[COUNT], sz[COUNT];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    pose_point<ESP>(a, R, u < count ? j0 + u * stride : a.M, b[u], x[u], y[u], z[u], w[u]);
+  for (int u = 0; u < COUNT; ++u) {
+    pose_point<ESP>(a, R, j0 + u * LPP, b[u], x[u], y[u], z[u], w[u]);
     sg[u] = sx[u] = sy[u] = sz[u] = 0.f;
   }
+#pragma unroll UNR
   for (int i = 0; i < a.N; ++i) {
     const float4 p = a.sPd[2 * i], r = a.sPd[2 * i + 1];
     float qc = 0.f;
     if (ESP) qc = a.sQd[i].x;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float w0 = plain ? __fsub_rn(r.z, w[u]) : r.z;
-      float E = __fmaf_rn(p.x, x[u], __fmaf_rn(p.z, y[u], __fmaf_rn(r.x, z[u], w0)));
+    for (int u = 0; u < COUNT; ++u) {
+      float E = __fmaf_rn(p.x, x[u],
+                          __fmaf_rn(p.z, y[u], __fmaf_rn(r.x, z[u], __fsub_rn(r.z, w[u]))));
       if (ESP) E = __fmaf_rn(qc, b[u].w, E);
       const float g = ex2(E);
       sg[u] = __fadd_rn(sg[u], g);
@@ -273,27 +273,93 @@ __device__ __noinline__ void far_points(const ShapeArgs& a, const Rot& R, int j0
     }
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    if (u >= count || j0 + u * stride >= a.M) continue;
-    const float s = plain ? 1.f : ex2(-w[u]);
-    add_point(acc, a.inv2k, b[u], x[u], y[u], z[u], __fmul_rn(sg[u], s), __fmul_rn(sx[u], s),
-              __fmul_rn(sy[u], s), __fmul_rn(sz[u], s));
+  for (int u = 0; u < COUNT; ++u)
+    if (j0 + u * LPP < a.M)
+      add_point(acc, a.inv2k, b[u], x[u], y[u], z[u], sg[u], sx[u], sy[u], sz[u]);
+}
+
+// Fit points of a lane in the reference frame: NP f32x2 pairs and an odd one.
+template <int NP>
+struct TilePoints {
+  static constexpr int kPairs = NP > 0 ? NP : 1;
+  float2 x[kPairs], y[kPairs], z[kPairs], c[kPairs], w[kPairs];
+  float ox, oy, oz, oc, ow;
+};
+
+// One loop over the reference points for pairs V0 .. V0 + NP of a tile with the factored
+// exponent, and (PL) its odd point with the unfactored one, which needs no 2^-w.
+template <int LPP, bool ESP, int V0, int NP, bool PL, int UNR, int TP>
+__device__ __forceinline__ void near_points(const ShapeArgs& a, const TilePoints<TP>& t, int j0,
+                                            Moments& acc) {
+  constexpr int T = 2 * NP + (PL ? 1 : 0);
+  float2 sg[NP > 0 ? NP : 1], sx[NP > 0 ? NP : 1], sy[NP > 0 ? NP : 1], sz[NP > 0 ? NP : 1];
+  float og = 0.f, ogx = 0.f, ogy = 0.f, ogz = 0.f;
+#pragma unroll
+  for (int v = 0; v < NP; ++v) sg[v] = sx[v] = sy[v] = sz[v] = f2(0.f, 0.f);
+#pragma unroll UNR
+  for (int i = 0; i < a.N; ++i) {
+    const float4 p = a.sPd[2 * i], r = a.sPd[2 * i + 1];
+    const float2 PX = f2(p.x, p.y), PY = f2(p.z, p.w), PZ = f2(r.x, r.y), PW = f2(r.z, r.w);
+    float2 QC;
+    if (ESP) QC = a.sQd[i];
+#pragma unroll
+    for (int v = 0; v < NP; ++v) {
+      float2 E = __ffma2_rn(PX, t.x[V0 + v],
+                            __ffma2_rn(PY, t.y[V0 + v], __ffma2_rn(PZ, t.z[V0 + v], PW)));
+      if (ESP) E = __ffma2_rn(QC, t.c[V0 + v], E);
+      const float2 g = f2(ex2(E.x), ex2(E.y));
+      sg[v] = __fadd2_rn(sg[v], g);
+      sx[v] = __ffma2_rn(g, PX, sx[v]);
+      sy[v] = __ffma2_rn(g, PY, sy[v]);
+      sz[v] = __ffma2_rn(g, PZ, sz[v]);
+    }
+    if (PL) {
+      float E = __fmaf_rn(PX.x, t.ox,
+                          __fmaf_rn(PY.x, t.oy, __fmaf_rn(PZ.x, t.oz, __fsub_rn(PW.x, t.ow))));
+      if (ESP) E = __fmaf_rn(QC.x, t.oc, E);
+      const float g = ex2(E);
+      og = __fadd_rn(og, g);
+      ogx = __fmaf_rn(g, PX.x, ogx);
+      ogy = __fmaf_rn(g, PY.x, ogy);
+      ogz = __fmaf_rn(g, PZ.x, ogz);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < T; ++u) {
+    const int j = j0 + (2 * V0 + u) * LPP;
+    if (j < a.M) {
+      const float4 b = a.sB[j];
+      if (PL && u == T - 1) {
+        add_point(acc, a.inv2k, b, t.ox, t.oy, t.oz, og, ogx, ogy, ogz);
+      } else {
+        const int v = u / 2, f = V0 + v;
+        const bool h = u % 2;
+        const float s = ex2(-(h ? t.w[f].y : t.w[f].x));
+        add_point(acc, a.inv2k, b, h ? t.x[f].y : t.x[f].x, h ? t.y[f].y : t.y[f].x,
+                  h ? t.z[f].y : t.z[f].x, __fmul_rn(h ? sg[v].y : sg[v].x, s),
+                  __fmul_rn(h ? sx[v].y : sx[v].x, s), __fmul_rn(h ? sy[v].y : sy[v].x, s),
+                  __fmul_rn(h ? sz[v].y : sz[v].x, s));
+      }
+    }
   }
 }
 
-// One loop over the reference points for NP f32x2 pairs of fit points per lane with the
-// factored exponent, and an odd point (PL) with the unfactored one, which needs no 2^-w.
-// GROUP points are voted together: a group with a far point (k |b'|^2 beyond kFactorMax in any
-// lane of the pose) is unfactored as a whole, and the pose's whole tile then takes far_points.
-template <int LPP, bool ESP, int NP, bool PL, int GROUP, int UNR>
+// A register tile: NP pairs of fit points per lane and an odd point (PL).  GROUP points are voted
+// together: a group with a far point (k |b'|^2 beyond kFactorMax in any lane of the pose) is
+// unfactored as a whole.  Molecules and surfaces longer than about 25 A have such poses at every
+// step, so this path runs as many points as the tile has, inline.  A tile of one group takes
+// far_points with all its points; in a tile of two groups the poses of a warp can be far in the
+// one, the other or both, so as soon as one is, the groups run one after the other: a warp then has
+// two ways to go at a time, not four.  One B200, molecules of 15-50 atoms stretched to 31 A, 50 x
+// 100, align_kernel -> here: 1024 pairs 4.88 -> 4.29 ms (8 lanes), 5.10 -> 4.30 (16 lanes); 2048 ESP
+// pairs 11.4 -> 10.6 ms (4 lanes).  An out-of-line function for four points, padded to that many
+// and taken by the whole tile, ran them in 6.92, 9.51 and 13.7 ms.
+template <int LPP, bool ESP, int NP, bool PL, int GROUP, int UNR, int FAR>
 __device__ __forceinline__ void pose_tile(const ShapeArgs& a, const Rot& R, int j0, Moments& acc) {
   constexpr int T = 2 * NP + (PL ? 1 : 0);
   constexpr int NG = (2 * NP + GROUP - 1) / GROUP;
-  float2 bx[NP > 0 ? NP : 1], by[NP > 0 ? NP : 1], bz[NP > 0 ? NP : 1], bc[NP > 0 ? NP : 1],
-      bw[NP > 0 ? NP : 1];
-  float2 sg[NP > 0 ? NP : 1], sx[NP > 0 ? NP : 1], sy[NP > 0 ? NP : 1], sz[NP > 0 ? NP : 1];
-  float ox = 0.f, oy = 0.f, oz = 0.f, oc = 0.f, ow = 0.f;   // the odd point
-  float og = 0.f, ogx = 0.f, ogy = 0.f, ogz = 0.f;
+  static_assert(NG <= 2, "one or two groups a tile");
+  TilePoints<NP> t;
   bool far[NG > 0 ? NG : 1] = {};
 #pragma unroll
   for (int v = 0; v < NP; ++v) {
@@ -306,105 +372,64 @@ __device__ __forceinline__ void pose_tile(const ShapeArgs& a, const Rot& R, int 
       c[h] = b.w;
       far[2 * v / GROUP] = far[2 * v / GROUP] || (j < a.M && w[h] > kFactorMax);
     }
-    bx[v] = f2(x[0], x[1]); by[v] = f2(y[0], y[1]); bz[v] = f2(z[0], z[1]);
-    bc[v] = f2(c[0], c[1]); bw[v] = f2(w[0], w[1]);
-    sg[v] = sx[v] = sy[v] = sz[v] = f2(0.f, 0.f);
+    t.x[v] = f2(x[0], x[1]); t.y[v] = f2(y[0], y[1]); t.z[v] = f2(z[0], z[1]);
+    t.c[v] = f2(c[0], c[1]); t.w[v] = f2(w[0], w[1]);
   }
   if (PL) {
     float4 b;
     const int j = j0 + 2 * NP * LPP;
-    pose_point<ESP>(a, R, j, b, ox, oy, oz, ow);
-    oc = b.w;
-    ow = j < a.M ? ow : INFINITY;
+    pose_point<ESP>(a, R, j, b, t.ox, t.oy, t.oz, t.ow);
+    t.oc = b.w;
+    t.ow = j < a.M ? t.ow : INFINITY;
   }
-  if (NP > 0) {
+  if constexpr (NG > 0) {
     // vote of this pose's lanes only: its path must not depend on the poses it shares a warp with
     const unsigned own = LPP >= 32 ? 0xffffffffu
                                    : ((1u << (LPP & 31)) - 1u) << ((threadIdx.x & 31) & ~(LPP - 1));
-    unsigned any = 0;
+    unsigned any = 0;   // in any pose of the warp
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
-      const unsigned vote = __ballot_sync(0xffffffffu, far[g]) & own;
-      far[g] = vote != 0;
+      const unsigned vote = __ballot_sync(0xffffffffu, far[g]);
+      far[g] = (vote & own) != 0;
       any |= vote;
     }
-    if (any) {
-      const ShapeArgs a2 = a;
-      const Rot R2 = R;
-      Moments m = acc;
-#pragma unroll
-      for (int u = 0; u < 2 * NP; u += 4)
-        far_points<ESP>(a2, R2, j0 + u * LPP, LPP, 2 * NP - u < 4 ? 2 * NP - u : 4,
-                        far[u / GROUP], m);
-      if (PL) far_points<ESP>(a2, R2, j0 + 2 * NP * LPP, LPP, 1, true, m);
-      acc = m;
+    if constexpr (NG == 1) {
+      if (far[0]) {
+        far_points<LPP, ESP, T, FAR>(a, R, j0, acc);
+        return;
+      }
+    } else if (any) {
+      constexpr int kRest = 2 * NP - GROUP;
+      if (far[0]) far_points<LPP, ESP, GROUP, FAR>(a, R, j0, acc);
+      else near_points<LPP, ESP, 0, GROUP / 2, false, UNR>(a, t, j0, acc);
+      __syncwarp();
+      if (far[1]) far_points<LPP, ESP, kRest, FAR>(a, R, j0 + GROUP * LPP, acc);
+      else near_points<LPP, ESP, GROUP / 2, kRest / 2, false, UNR>(a, t, j0, acc);
+      if (PL) far_points<LPP, ESP, 1, FAR>(a, R, j0 + 2 * NP * LPP, acc);
       return;
     }
   }
-#pragma unroll UNR
-  for (int i = 0; i < a.N; ++i) {
-    const float4 p = a.sPd[2 * i], r = a.sPd[2 * i + 1];
-    const float2 PX = f2(p.x, p.y), PY = f2(p.z, p.w), PZ = f2(r.x, r.y), PW = f2(r.z, r.w);
-    float2 QC;
-    if (ESP) QC = a.sQd[i];
-#pragma unroll
-    for (int v = 0; v < NP; ++v) {
-      float2 E = __ffma2_rn(PX, bx[v], __ffma2_rn(PY, by[v], __ffma2_rn(PZ, bz[v], PW)));
-      if (ESP) E = __ffma2_rn(QC, bc[v], E);
-      const float2 g = f2(ex2(E.x), ex2(E.y));
-      sg[v] = __fadd2_rn(sg[v], g);
-      sx[v] = __ffma2_rn(g, PX, sx[v]);
-      sy[v] = __ffma2_rn(g, PY, sy[v]);
-      sz[v] = __ffma2_rn(g, PZ, sz[v]);
-    }
-    if (PL) {
-      float E = __fmaf_rn(PX.x, ox, __fmaf_rn(PY.x, oy, __fmaf_rn(PZ.x, oz, __fsub_rn(PW.x, ow))));
-      if (ESP) E = __fmaf_rn(QC.x, oc, E);
-      const float g = ex2(E);
-      og = __fadd_rn(og, g);
-      ogx = __fmaf_rn(g, PX.x, ogx);
-      ogy = __fmaf_rn(g, PY.x, ogy);
-      ogz = __fmaf_rn(g, PZ.x, ogz);
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < T; ++u) {
-    const int j = j0 + u * LPP;
-    if (j < a.M) {
-      const float4 b = a.sB[j];
-      if (PL && u == T - 1) {
-        add_point(acc, a.inv2k, b, ox, oy, oz, og, ogx, ogy, ogz);
-      } else {
-        const int v = u / 2;
-        const bool h = u % 2;
-        const float s = ex2(-(h ? bw[v].y : bw[v].x));
-        add_point(acc, a.inv2k, b, h ? bx[v].y : bx[v].x, h ? by[v].y : by[v].x,
-                  h ? bz[v].y : bz[v].x, __fmul_rn(h ? sg[v].y : sg[v].x, s),
-                  __fmul_rn(h ? sx[v].y : sx[v].x, s), __fmul_rn(h ? sy[v].y : sy[v].x, s),
-                  __fmul_rn(h ? sz[v].y : sz[v].x, s));
-      }
-    }
-  }
+  near_points<LPP, ESP, 0, NP, PL, UNR>(a, t, j0, acc);
 }
 
 // All fit points of a pose: register tiles of GROUP points per lane, the last of them together
 // with points left over (TAIL at most).
-template <int LPP, bool ESP, int GROUP, int TAIL, int UNR>
+template <int LPP, bool ESP, int GROUP, int TAIL, int UNR, int FAR>
 __device__ __forceinline__ void pose_sums(const ShapeArgs& a, const Rot& R, int lane,
                                           Moments& acc) {
   int left = (a.M + LPP - 1) / LPP;   // points per lane
   int j = lane;
   for (; left > TAIL; left -= GROUP, j += GROUP * LPP)
-    pose_tile<LPP, ESP, GROUP / 2, false, GROUP, UNR>(a, R, j, acc);
+    pose_tile<LPP, ESP, GROUP / 2, false, GROUP, UNR, FAR>(a, R, j, acc);
   switch (left) {
-    case 1: pose_tile<LPP, ESP, 0, true, GROUP, UNR>(a, R, j, acc); break;
-    case 2: pose_tile<LPP, ESP, 1, false, GROUP, UNR>(a, R, j, acc); break;
-    case 3: pose_tile<LPP, ESP, 1, true, GROUP, UNR>(a, R, j, acc); break;
-    case 4: pose_tile<LPP, ESP, 2, false, GROUP, UNR>(a, R, j, acc); break;
-    case 5: if (TAIL >= 5) pose_tile<LPP, ESP, 2, true, GROUP, UNR>(a, R, j, acc); break;
-    case 6: if (TAIL >= 6) pose_tile<LPP, ESP, 3, false, GROUP, UNR>(a, R, j, acc); break;
-    case 7: if (TAIL >= 7) pose_tile<LPP, ESP, 3, true, GROUP, UNR>(a, R, j, acc); break;
-    case 8: if (TAIL >= 8) pose_tile<LPP, ESP, 4, false, GROUP, UNR>(a, R, j, acc); break;
+    case 1: pose_tile<LPP, ESP, 0, true, GROUP, UNR, FAR>(a, R, j, acc); break;
+    case 2: pose_tile<LPP, ESP, 1, false, GROUP, UNR, FAR>(a, R, j, acc); break;
+    case 3: pose_tile<LPP, ESP, 1, true, GROUP, UNR, FAR>(a, R, j, acc); break;
+    case 4: pose_tile<LPP, ESP, 2, false, GROUP, UNR, FAR>(a, R, j, acc); break;
+    case 5: if (TAIL >= 5) pose_tile<LPP, ESP, 2, true, GROUP, UNR, FAR>(a, R, j, acc); break;
+    case 6: if (TAIL >= 6) pose_tile<LPP, ESP, 3, false, GROUP, UNR, FAR>(a, R, j, acc); break;
+    case 7: if (TAIL >= 7) pose_tile<LPP, ESP, 3, true, GROUP, UNR, FAR>(a, R, j, acc); break;
+    case 8: if (TAIL >= 8) pose_tile<LPP, ESP, 4, false, GROUP, UNR, FAR>(a, R, j, acc); break;
     default: break;
   }
 }
@@ -420,13 +445,18 @@ __device__ __forceinline__ void pose_sums(const ShapeArgs& a, const Rot& R, int 
 //    shape + pharm pairs, 8 lanes: 34.5 ms with up to 4 points unrolled twice, 35.4 unrolled
 //    four times, 41.0 with up to 5 points; align_kernel 38.0).  A few pairs of 4 lanes (ALONE:
 //    their warps have a scheduler each) take up to 8: one pair of 30 atoms 553 us, 617 with 5.
+//    With last tiles of 8 points in every launch (GROUP 8) the loop is unrolled twice: 1024 pairs
+//    of 50 x 100, 4 lanes: 3.26 ms, 3.71 unrolled four times.  The loop of far points is unrolled
+//    where latency bounds it (ALONE, 16 and 32 lanes) and not in the many warps of 4 or 8 lanes
+//    (1024 stretched pairs, 4 lanes: 4.93 ms, 5.51 unrolled twice).
 template <int LPP, int MODE, int GROUP, bool ALONE>
 struct SpreadTile {
   static constexpr bool kTwo = MODE == FSS_MODE_SHAPE_PHARM || MODE == FSS_MODE_SHAPE_COLOR ||
                                MODE == FSS_MODE_PHARM;
   static constexpr int kRegs = kTwo ? 128 : 168;
   static constexpr int kTail = GROUP == 8 || ALONE ? 8 : kTwo || MODE == FSS_MODE_ESP_COMBO ? 4 : 5;
-  static constexpr int kUnroll = kTwo ? 2 : 4;
+  static constexpr int kUnroll = kTwo || GROUP == 8 ? 2 : 4;
+  static constexpr int kFarUnroll = LPP <= 8 && !ALONE ? 1 : 2;
 };
 
 template <int LPP, int MODE, int GROUP, int EXT, bool ALONE>
@@ -554,7 +584,7 @@ __global__ void __maxnreg__((SpreadTile<LPP, MODE, GROUP, ALONE>::kRegs))
           const ShapeArgs a{sP, sQc, sB, N, M, s.t[0], s.t[1], s.t[2], p.k, p.e, p.inv2k};
           Moments ms;
           ms.zero();
-          pose_sums<LPP, kEsp, GROUP, Tile::kTail, Tile::kUnroll>(a, R, lane, ms);
+          pose_sums<LPP, kEsp, GROUP, Tile::kTail, Tile::kUnroll, Tile::kFarUnroll>(a, R, lane, ms);
           rs.from(ms, s.q);
           S::reduce(rs, lane, os);
           S::scale(os, lane, p.Kc, p.aKc);
