@@ -25,6 +25,7 @@ from typing import Optional, Sequence
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from . import align as al
 from . import kernels as K
@@ -242,6 +243,7 @@ def _align_device_once(mode, ref: Optional[CloudSet], fit: Optional[CloudSet],
         shift = None
         if mode == "pharm":
             _, g_ref, shift = _centred_pharm(ref_ph)
+            shift = shift.detach()
             g_fit = _centred_pharm(fit_ph)[1]
         elif mode in ESP_COMBO_MODES:
             g_ref, g_fit = tile["ref_surf"], tile["fit_surf"]
@@ -298,7 +300,12 @@ def _align_device_once(mode, ref: Optional[CloudSet], fit: Optional[CloudSet],
                               pharm_extended=al.extended_code(extended_points, only_extended),
                               **tile)
         sc, q, t = res
-        out = al.AlignResult((sc, q, K.fold_centroids(q, t, pair_ref, pair_fit, c_ref, c_fit)))
+        if _differentiated(c_ref) or _differentiated(c_fit):
+            t = (t - torch.einsum("bij,bj->bi", al._quat_rot(q), c_fit[pair_fit.long()])
+                 + c_ref[pair_ref.long()])
+        else:
+            t = K.fold_centroids(q, t, pair_ref, pair_fit, c_ref, c_fit)
+        out = al.AlignResult((sc, q, t))
         out.rows = res.rows
         return out
     if seeds is None:
@@ -313,9 +320,24 @@ def _align_device_once(mode, ref: Optional[CloudSet], fit: Optional[CloudSet],
 
 def _centred_pharm(ps: PharmSet):
     """The set with every molecule's anchors centred on its own centroid (types kept), the centred
-    anchors as a plain cloud (for seeding), and the centroids."""
+    anchors as a plain cloud (for seeding), and the centroids.  The poses do not depend on the
+    anchors for autograd; the centroids folded into the translations do, so anchors that carry a
+    gradient or a tangent get their centroids from torch."""
     if ps.anc.dtype != torch.float32:
         raise ValueError("mode 'pharm' re-centres its anchors: it needs float32 sets")
     anc, pts, c = K.centre_anchors(ps)
+    if _differentiated(ps.anc):
+        n = (ps.off[1:] - ps.off[:-1]).long()[:, None]
+        ar = torch.arange(max(int(ps.max_points), 1), device=c.device)
+        rows = torch.where(ar < n, ps.off[:-1, None] + ar, 0)
+        xyz = ps.anc[:, :3]
+        padded = xyz[rows] if len(xyz) else xyz.new_zeros(*rows.shape, 3)
+        c = torch.where((ar < n)[..., None], padded, 0.0).sum(1) / n.clamp(min=1)
     return (PharmSet(anc, ps.vec, ps.off, ps.counts, ps.max_points),
             CloudSet(pts, ps.off, ps.counts, ps.max_points), c)
+
+
+def _differentiated(t: torch.Tensor) -> bool:
+    """Whether autograd follows ``t``: backwards, or forwards as a dual tensor."""
+    return ((t.requires_grad and torch.is_grad_enabled())
+            or forward_ad.unpack_dual(t).tangent is not None)
