@@ -57,7 +57,10 @@ class PackedTanimoto(torch.autograd.Function):
         unit = None
         if (grad_on and need[1] and not need[0] and 0 < max_fit <= UNIT_POINTS
                 and max_ref <= UNIT_POINTS and 16 * P * int(max_fit) <= UNIT_BYTES):
-            unit = torch.empty(P, int(max_fit), 4, dtype=_f32, device=dev)
+            try:
+                unit = torch.empty(P, int(max_fit), 4, dtype=_f32, device=dev)
+            except torch.OutOfMemoryError:   # the backward then evaluates the Gaussians again
+                pass
         args = (ptr(ref_pts, _f32), ptr(ref_off, _i32), ptr(fit_pts, _f32), ptr(fit_off, _i32),
                 ptr(pair_ref, _i32), ptr(pair_fit, _i32), P, int(max_ref), int(max_fit),
                 float(alpha), int(esp), float(inv_lam), ptr(score), ptr(ov))
