@@ -122,40 +122,35 @@ def candidates(mode: str, max_fit: int, n_starts: int, tensor_cores: bool = None
             continue  # a pose per 1-2 lanes pays off only for small molecules in large batches
         if mode == "pharm" and lpp > 8:
             continue
+        # Start blocks are always named: with 0 the library chooses them from the number of pairs,
+        # and a sample of the batch could be timed with other blocks than the batch then runs.
+        # The fewest idle pose slots; smaller CTAs (twice the blocks): less waiting at the
+        # per-item barrier; and blocks that fill whole warps (no lanes shadow an idle start except
+        # in a pair's last block) in CTAs of 1, 2 or 4 warps, which spread evenly over the SM's
+        # four schedulers.  A 5-warp CTA puts two warps on one scheduler, and its other warps then
+        # wait ~24 % of the time at the per-item barrier (measured on 200-400 point surfaces).
+        base = _fewest_idle(lpp, n_starts)
+        blocks = [base, 2 * base] + [-(-n_starts // (warps * (32 // lpp))) for warps in (1, 2, 4)]
+        blocks = [c for c in dict.fromkeys(blocks) if c <= n_starts]
         for var in variants:
-            for cps in (0, 2, 1):   # 0 = as many CTAs per SM as fit
-                out.append({"lanes_per_pose": lpp, "chunks": 0, "cta_per_sm": cps,
-                            "kernel_variant": var})
-            # smaller CTAs (twice the default start blocks): less waiting at the per-item barrier
-            base = _auto_chunks(lpp, n_starts)
-            if 2 * base <= n_starts:
-                out.append({"lanes_per_pose": lpp, "chunks": 2 * base, "cta_per_sm": 0,
-                            "kernel_variant": var})
-            # start blocks that fill whole warps (no lanes shadow an idle start except in a
-            # pair's last block), in CTAs of 1, 2 or 4 warps: CTAs whose warps spread evenly
-            # over the SM's four schedulers.  A 5-warp CTA puts two warps on one scheduler,
-            # and its other warps then wait ~24 % of the time at the per-item barrier
-            # (measured on 200-400 point surfaces).
-            for warps in ((1, 2, 4) if max_fit < 64 else (2, 4)):
-                ppc = warps * (32 // lpp)
-                ch = -(-n_starts // ppc)
-                if ch not in (base, 2 * base) and ch <= n_starts:
-                    out.append({"lanes_per_pose": lpp, "chunks": ch, "cta_per_sm": 0,
+            for ch in blocks:
+                for cps in ((0, 2, 1) if ch == base else (0,)):   # 0 = as many CTAs as fit
+                    out.append({"lanes_per_pose": lpp, "chunks": ch, "cta_per_sm": cps,
                                 "kernel_variant": var})
     if tensor_cores and mode in ("shape", "esp") and max_fit >= 16:
-        base = _auto_chunks(32, n_starts)
+        base = _fewest_idle(32, n_starts)
         ch4 = -(-n_starts // 4)     # one pose per warp: CTAs of 4 warps
         for acc in (2, 3):
-            for ch, cps in ((0, 0), (0, 1), (2 * base, 0), (ch4, 0)):
+            for ch, cps in dict.fromkeys(((base, 0), (base, 1), (2 * base, 0), (ch4, 0))):
                 if ch <= n_starts:
                     out.append({"lanes_per_pose": 32, "chunks": ch, "cta_per_sm": cps,
                                 "accumulate": acc})
     return out
 
 
-def _auto_chunks(lpp: int, n_starts: int, max_threads: int = 320) -> int:
-    """The library's default start-block count for a lanes-per-pose choice: the fewest idle
-    pose slots with CTAs of at most max_threads threads (fss_align.cu auto_tile)."""
+def _fewest_idle(lpp: int, n_starts: int, max_threads: int = 320) -> int:
+    """The start-block count with the fewest idle pose slots in CTAs of at most max_threads threads
+    (auto_chunks in fss_align.cu: what the library keeps for launches of less than two rounds)."""
     best_c, best_w = 1, 1 << 30
     for c in range(1, n_starts + 1):
         ppc = -(-n_starts // c)
