@@ -11,7 +11,8 @@ Tunables of one launch (``fss_align_desc``):
                   32 lanes per pose)
   kernel_variant  code variant of the FP32-lane loop (shape/ESP modes): 1 base, 2 wide
                   register tile, 3 one-CTA/SM register budget, 4 base tile unrolled 4x,
-                  5 eight-point register tile (small molecules)
+                  5 eight-point register tile (small molecules); where the optimiser state is
+                  spread over a pose's lanes, 1 and 3 are one kernel and are tried once
 
 For a new problem shape the tuner times each candidate on a sample of the batch's pairs
 (the costliest and a spread of the rest) for a few Adam steps, with CUDA events, and keeps
@@ -133,6 +134,8 @@ def candidates(mode: str, max_fit: int, n_starts: int, tensor_cores: bool = None
         blocks = [base, 2 * base] + [-(-n_starts // (warps * (32 // lpp))) for warps in (1, 2, 4)]
         blocks = [c for c in dict.fromkeys(blocks) if c <= n_starts]
         for var in variants:
+            if var == 3 and _same_kernel(mode, lpp, max_fit):
+                continue
             for ch in blocks:
                 for cps in ((0, 2, 1) if ch == base else (0,)):   # 0 = as many CTAs as fit
                     out.append({"lanes_per_pose": lpp, "chunks": ch, "cta_per_sm": cps,
@@ -146,6 +149,12 @@ def candidates(mode: str, max_fit: int, n_starts: int, tensor_cores: bool = None
                     out.append({"lanes_per_pose": 32, "chunks": ch, "cta_per_sm": cps,
                                 "accumulate": acc})
     return out
+
+
+def _same_kernel(mode: str, lpp: int, max_fit: int) -> bool:
+    """Whether variants 1 and 3 launch one kernel: spread_kernel, which takes only the register tile
+    (4 fit points a lane in both) from the variant (launch_align in fss_align_kernel.cuh)."""
+    return lpp >= 4 and max_fit <= 16 * lpp and not (mode == "esp" and lpp == 32)
 
 
 def _fewest_idle(lpp: int, n_starts: int, max_threads: int = 320) -> int:

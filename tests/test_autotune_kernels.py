@@ -23,3 +23,15 @@ def test_start_blocks_are_named(mode, max_fit, starts):
         assert min(fit, key=lambda c: (idle(c), c)) in mine
         for warps in (1, 2, 4):
             assert -(-starts // (warps * 32 // lanes)) in mine
+
+
+@pytest.mark.parametrize("mode,max_fit,starts", SIZES)
+def test_each_kernel_once(mode, max_fit, starts):
+    def kernel(c):   # launch_align: from 4 lanes on, up to 16 fit points a lane, 1 and 3 are one
+        lanes, var = c["lanes_per_pose"], c.get("kernel_variant", 0)
+        spread = lanes >= 4 and max_fit <= 16 * lanes
+        if var == 3 and spread and not (mode == "esp" and lanes == 32):
+            var = 1
+        return lanes, c["chunks"], c["cta_per_sm"], var, c.get("accumulate", 0)
+    tiles = [kernel(c) for c in autotune.candidates(mode, max_fit, starts, tensor_cores=True)]
+    assert len(tiles) == len(set(tiles))
