@@ -17,7 +17,7 @@ Tunables of one launch (``fss_align_desc``):
 For a new problem shape the tuner times each candidate on a sample of the batch's pairs
 (the costliest and a spread of the rest) for a few Adam steps, with CUDA events, and keeps
 the fastest.  Results are cached per (device, mode, size buckets, starts, pair bucket, step-count
-class) in memory and in a JSON file (``$FSS_AUTOTUNE_CACHE`` or ``~/.cache/fast_shepherd_score_b200/autotune.json``).
+class, kernel revision) in memory and in a JSON file (``$FSS_AUTOTUNE_CACHE`` or ``~/.cache/fast_shepherd_score_b200/autotune.json``).
 Set ``FSS_AUTOTUNE=0`` to disable tuning (the library's built-in default is then used).
 """
 from __future__ import annotations
@@ -35,6 +35,9 @@ _LOCK = threading.Lock()
 _MEM: dict = {}
 _LOADED = False
 LANES = (1, 2, 4, 8, 16, 32)
+# Revision of the kernels behind a tile, part of the key: a cached ranking of other kernels is not
+# used.  Raised whenever a change to them can change which tile is the fastest.
+KERNELS = 2
 
 
 def _cache_path() -> str:
@@ -100,7 +103,7 @@ def shape_key(device, mode: str, max_ref: int, max_fit: int, mean_fit: float, n_
               n_pairs: int, steps: int = 200) -> str:
     name = _device_name(device)
     return (f"{name}|{mode}|r{_bucket(max_ref)}|f{_bucket(max_fit)}|m{_bucket(int(mean_fit))}"
-            f"|s{n_starts}|p{_bucket(n_pairs)}|t{steps_class(steps)}")
+            f"|s{n_starts}|p{_bucket(n_pairs)}|t{steps_class(steps)}|k{KERNELS}")
 
 
 def candidates(mode: str, max_fit: int, n_starts: int, tensor_cores: bool = None):

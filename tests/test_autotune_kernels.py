@@ -35,3 +35,11 @@ def test_each_kernel_once(mode, max_fit, starts):
         return lanes, c["chunks"], c["cta_per_sm"], var, c.get("accumulate", 0)
     tiles = [kernel(c) for c in autotune.candidates(mode, max_fit, starts, tensor_cores=True)]
     assert len(tiles) == len(set(tiles))
+
+
+def test_key_names_the_kernels(monkeypatch):
+    monkeypatch.setattr(autotune, "_device_name", lambda device: "gpu")
+    key = lambda: autotune.shape_key("cuda:0", "shape", 50, 50, 30.0, 50, 256, 200)
+    before = key()
+    monkeypatch.setattr(autotune, "KERNELS", autotune.KERNELS + 1)
+    assert key() != before
