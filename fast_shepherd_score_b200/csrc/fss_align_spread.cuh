@@ -435,10 +435,14 @@ __device__ __forceinline__ void pose_sums(const ShapeArgs& a, const Rot& R, int 
 }
 
 // Registers, the largest last tile and the unroll of a tile's loop.  168 registers keep 12 warps
-// on an SM, 128 keep 16.
-//  * shape, ESP, ESP combo: 168 -- with a few rounds of CTAs the largest pair's serial chain of
-//    steps decides the time, and runs faster beside 11 warps than beside 15 (256 pairs of 15-50
-//    atoms, 8 lanes: 1.56 ms, 2.0 ms at 128 registers; combo 2.04 and 2.27 ms);
+// on an SM, 128 keep 16, 96 keep 20.
+//  * shape, ESP: 168 -- with a few rounds of CTAs the largest pair's serial chain of steps decides
+//    the time, and runs faster beside 11 warps than beside 15 (256 pairs of 15-50 atoms, 8 lanes:
+//    1.56 ms, 2.0 ms at 128 registers);
+//  * ESP combo: 96 -- its field points are spread over all lanes and wait for each other's rsqrt
+//    and ex2, so warps count (8 x 60, 16 lanes, at 168 / 128 / 96 registers: 256 pairs 1.08 / 1.04 /
+//    1.03 ms, 4096 pairs 8.51 / 7.93 / 7.80; align_kernel at 96: 1.10 and 8.08), and
+//    128 for a few pairs (64 pairs, 4 lanes: 2.60 / 2.49 / 2.48);
 //  * two channels, pharmacophores: 128 (16 384 pairs of 20 x 100: 24.8 ms, 25.9 ms at 168);
 //  * last tiles of up to 5 points, 4 with a second channel beside them: the warps of ragged pairs
 //    run different tiles, and more of them, or longer loops, miss the instruction cache (8192
@@ -453,7 +457,8 @@ template <int LPP, int MODE, int GROUP, bool ALONE>
 struct SpreadTile {
   static constexpr bool kTwo = MODE == FSS_MODE_SHAPE_PHARM || MODE == FSS_MODE_SHAPE_COLOR ||
                                MODE == FSS_MODE_PHARM;
-  static constexpr int kRegs = kTwo ? 128 : 168;
+  static constexpr int kRegs =
+      kTwo ? 128 : MODE != FSS_MODE_ESP_COMBO ? 168 : ALONE ? 128 : 96;
   static constexpr int kTail = GROUP == 8 || ALONE ? 8 : kTwo || MODE == FSS_MODE_ESP_COMBO ? 4 : 5;
   static constexpr int kUnroll = kTwo || GROUP == 8 ? 2 : 4;
   static constexpr int kFarUnroll = LPP <= 8 && !ALONE ? 1 : 2;
