@@ -452,7 +452,8 @@ __device__ __forceinline__ void pose_sums(const ShapeArgs& a, const Rot& R, int 
 //    With last tiles of 8 points in every launch (GROUP 8) the loop is unrolled twice: 1024 pairs
 //    of 50 x 100, 4 lanes: 3.26 ms, 3.71 unrolled four times.  The loop of far points is unrolled
 //    where latency bounds it (ALONE, 16 and 32 lanes) and not in the many warps of 4 or 8 lanes
-//    (1024 stretched pairs, 4 lanes: 4.93 ms, 5.51 unrolled twice).
+//    (1024 stretched pairs, 4 lanes: 4.93 ms, 5.51 unrolled twice); two channels at 8 lanes unroll
+//    it for the compact molecules beside it (16 384 pairs of 20 x 100: 27.5 ms, 28.0 without).
 template <int LPP, int MODE, int GROUP, bool ALONE>
 struct SpreadTile {
   static constexpr bool kTwo = MODE == FSS_MODE_SHAPE_PHARM || MODE == FSS_MODE_SHAPE_COLOR ||
@@ -461,7 +462,7 @@ struct SpreadTile {
       kTwo ? 128 : MODE != FSS_MODE_ESP_COMBO ? 168 : ALONE ? 128 : 96;
   static constexpr int kTail = GROUP == 8 || ALONE ? 8 : kTwo || MODE == FSS_MODE_ESP_COMBO ? 4 : 5;
   static constexpr int kUnroll = kTwo || GROUP == 8 ? 2 : 4;
-  static constexpr int kFarUnroll = LPP <= 8 && !ALONE ? 1 : 2;
+  static constexpr int kFarUnroll = LPP <= (kTwo ? 4 : 8) && !ALONE ? 1 : 2;
 };
 
 template <int LPP, int MODE, int GROUP, int EXT, bool ALONE>
