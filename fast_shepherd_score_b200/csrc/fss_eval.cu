@@ -38,18 +38,18 @@ __device__ __forceinline__ void expand_point(float ax, float ay, float az, float
 
 }  // namespace
 
-// A pose to a CTA of one warp (atom clouds) or two (surfaces).  A surface is bound by the pairwise
-// loop's ex2 and FP32 and wants more warps than one per pose; an atom cloud by the instructions and
-// latency around a short loop, where a second warp, or several poses to a warp, gave nothing.  The
-// reduction halves the components with the lanes (LanePose), 13 shuffles for 40.  One B200, before
+// A pose to a CTA of one warp (atom clouds) or two (surfaces, few poses).  A surface is bound by the
+// pairwise loop's ex2 and FP32 and wants more warps than one per pose; an atom cloud by the
+// instructions and latency around a short loop, where a second warp, or several poses to a warp, gave
+// nothing.  The reduction halves the components with the lanes (LanePose), 13 shuffles for 40.  One B200, before
 // (a warp a pose, full butterflies) -> after: 1600 poses of 200-400 charged points 129 -> 87 us, 20
 // of them 72 -> 35; 12 800 poses of 15-50 atoms 20.3 -> 19.7, 100 of them 4.5 -> 4.2.
 template <bool ESP, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) overlap_eval_kernel(
     const float* __restrict__ A, const float* __restrict__ B, const float* __restrict__ CA,
     const float* __restrict__ CB, const float* __restrict__ q, const float* __restrict__ t,
-    const int* __restrict__ Nr, const int* __restrict__ Mr, int K, int Npad, int Mpad, float k,
-    float e, float inv2k, float Kc, float aKc, int need_grad, float* V, float* dQ, float* dT) {
+    const int* __restrict__ Nr, const int* __restrict__ Mr, int Npad, int Mpad, float k, float e,
+    float inv2k, float Kc, float aKc, int need_grad, float* V, float* dQ, float* dT) {
   constexpr int kThreads = 32 * WARPS;
   extern __shared__ __align__(16) float4 smem[];
   __shared__ float red[96];
@@ -247,17 +247,19 @@ int overlap_eval_launch(const float* A, const float* B, const float* CA, const f
   const float inv2k = (float)(1.0 / (a * 1.4426950408889634));
   const double Kd = std::pow(M_PI, 1.5) / std::pow(2.0 * a, 1.5);
   const size_t smem = sizeof(float4) * (2 * (size_t)Npad + Mpad + (esp ? (Npad + 1) / 2 : 0));
-  // Above 64 fit points each lane of two warps has a whole register tile: 1600 poses of 60-100
-  // charged points 12.7 us with one warp and 12.5 with two, of 200-400 points 129 and 87.  Below,
-  // lanes of the second warp would have no point.
-  const bool wide = Mpad > 64;
+  // Two warps from 256 fit points on, where each lane has whole register tiles, and above 64
+  // points (below, lanes of the second would have none) while the poses are few.  In us with one
+  // and with two: 148 poses of 65 points 4.5 and 3.8, 13 000 of them 24.3 and 35.4; of 100 points
+  // 6.5 and 5.1, 47.4 and 58.4; 600 charged poses of 200 points 19.1 and 16.5, 6000 72 and 88;
+  // 3000 of 300 points 92 and 77.
+  const bool wide = Mpad >= 256 || (Mpad > 64 && K <= 12 * num_sms());
   const auto kern = esp ? (wide ? overlap_eval_kernel<true, 2> : overlap_eval_kernel<true, 1>)
                         : (wide ? overlap_eval_kernel<false, 2> : overlap_eval_kernel<false, 1>);
   const cudaError_t ce =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ce != cudaSuccess)
     return set_error(FSS_ERR_CUDA, std::string("fss_overlap_grad: ") + cudaGetErrorString(ce));
-  kern<<<K, wide ? 64 : 32, smem, st>>>(A, B, CA, CB, q, t, Nr, Mr, K, Npad, Mpad, k, e, inv2k,
+  kern<<<K, wide ? 64 : 32, smem, st>>>(A, B, CA, CB, q, t, Nr, Mr, Npad, Mpad, k, e, inv2k,
                                         (float)Kd, (float)(a * Kd), need_grad, V, dQ, dT);
   return check_launch("fss_overlap_grad");
 }
