@@ -247,12 +247,12 @@ int overlap_eval_launch(const float* A, const float* B, const float* CA, const f
   const float inv2k = (float)(1.0 / (a * 1.4426950408889634));
   const double Kd = std::pow(M_PI, 1.5) / std::pow(2.0 * a, 1.5);
   const size_t smem = sizeof(float4) * (2 * (size_t)Npad + Mpad + (esp ? (Npad + 1) / 2 : 0));
-  // Two warps from 256 fit points on, where each lane has whole register tiles, and above 64
-  // points (below, lanes of the second would have none) while the poses are few.  In us with one
-  // and with two: 148 poses of 65 points 4.5 and 3.8, 13 000 of them 24.3 and 35.4; of 100 points
-  // 6.5 and 5.1, 47.4 and 58.4; 600 charged poses of 200 points 19.1 and 16.5, 6000 72 and 88;
-  // 3000 of 300 points 92 and 77.
-  const bool wide = Mpad >= 256 || (Mpad > 64 && K <= 12 * num_sms());
+  // Two warps from 256 fit points on, where each lane has whole register tiles, if the reference is
+  // no small one, and above 64 points (below, lanes of the second would have none) while the poses
+  // are few.  In us with one and with two: 148 poses of 65 points 4.5 and 3.8, 13 000 of them 24.3
+  // and 35.4; of 100 points 6.5 and 5.1, 47.4 and 58.4; 600 charged poses of 200 points 19.1 and
+  // 16.5, 6000 72 and 88; 3000 of 300 points 92 and 77; 13 000 of 400 against 30 points 48.8 and 55.3.
+  const bool wide = Mpad > 64 && ((Mpad >= 256 && Npad > 64) || K <= 12 * num_sms());
   const auto kern = esp ? (wide ? overlap_eval_kernel<true, 2> : overlap_eval_kernel<true, 1>)
                         : (wide ? overlap_eval_kernel<false, 2> : overlap_eval_kernel<false, 1>);
   const cudaError_t ce =

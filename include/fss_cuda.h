@@ -62,7 +62,7 @@ int fss_max_points(void);
  * A (K,N_pad,3), B (K,M_pad,3), CA (K,N_pad), CB (K,M_pad), q (K,4), t (K,3),
  * N_real/M_real (K) int32 (NULL = fully real).  Outputs V (K), dQ (K,4) = dV/dq,
  * dT (K,3) = dV/dt; dQ/dT untouched when need_grad == 0.  The order of a pose's sums depends on
- * M_pad and, from 65 to 255, on whether K exceeds 12 poses an SM: the same call gives the same
+ * M_pad and, above 64, on whether K exceeds 12 poses an SM: the same call gives the same
  * bits, the pose in a batch of another size the same value to rounding.
  * ------------------------------------------------------------------------------------- */
 int fss_overlap_grad(const float *A, const float *B, const float *CA, const float *CB,
