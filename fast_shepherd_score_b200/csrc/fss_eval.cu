@@ -44,7 +44,7 @@ __device__ __forceinline__ void expand_point(float ax, float ay, float az, float
 // nothing.  The reduction halves the components with the lanes (LanePose), 13 shuffles for 40.  One B200, before
 // (a warp a pose, full butterflies) -> after: 1600 poses of 200-400 charged points 129 -> 87 us, 20
 // of them 72 -> 35; 12 800 poses of 15-50 atoms 20.3 -> 19.7, 100 of them 4.5 -> 4.2.
-template <bool ESP, int WARPS>
+template <bool ESP, int WARPS, int UNR>
 __global__ void __launch_bounds__(32 * WARPS) overlap_eval_kernel(
     const float* __restrict__ A, const float* __restrict__ B, const float* __restrict__ CA,
     const float* __restrict__ CB, const float* __restrict__ q, const float* __restrict__ t,
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(32 * WARPS) overlap_eval_kernel(
   const Rot R = quat_to_rot(qq);
   Moments acc;
   acc.zero();
-  shape_pose<kThreads, ESP, 2, 4>(sP, sQ, sB, N, M, tid, R, t[row * 3] - c.x, t[row * 3 + 1] - c.y,
+  shape_pose<kThreads, ESP, 2, UNR>(sP, sQ, sB, N, M, tid, R, t[row * 3] - c.x, t[row * 3 + 1] - c.y,
                                   t[row * 3 + 2] - c.z, k, e, inv2k, acc);
   Reduced r;
   r.from(acc, qq);
@@ -253,8 +253,14 @@ int overlap_eval_launch(const float* A, const float* B, const float* CA, const f
   // and 35.4; of 100 points 6.5 and 5.1, 47.4 and 58.4; 600 charged poses of 200 points 19.1 and
   // 16.5, 6000 72 and 88; 3000 of 300 points 92 and 77; 13 000 of 400 against 30 points 48.8 and 55.3.
   const bool wide = Mpad > 64 && ((Mpad >= 256 && Npad > 64) || K <= 12 * num_sms());
-  const auto kern = esp ? (wide ? overlap_eval_kernel<true, 2> : overlap_eval_kernel<true, 1>)
-                        : (wide ? overlap_eval_kernel<false, 2> : overlap_eval_kernel<false, 1>);
+  // One warp: the loop unrolled twice instead of four times needs fewer registers (more poses on
+  // an SM) and pays for small clouds in large batches: 13 000 poses of 30 points 14.7 and 14.1 us,
+  // charged 17.1 and 16.0; 600 of 50 points 4.9 and 4.7.
+  const bool few = K <= (esp ? 16 : 24) * num_sms() || Npad > 100;
+  const auto kern = esp ? (wide ? overlap_eval_kernel<true, 2, 4>
+                           : few ? overlap_eval_kernel<true, 1, 4> : overlap_eval_kernel<true, 1, 2>)
+                        : (wide ? overlap_eval_kernel<false, 2, 4>
+                           : few ? overlap_eval_kernel<false, 1, 4> : overlap_eval_kernel<false, 1, 2>);
   const cudaError_t ce =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ce != cudaSuccess)

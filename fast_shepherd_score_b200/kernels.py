@@ -43,10 +43,15 @@ def _counts(x, device):
 
 
 def _pose_outputs(K, dev, need_grad):
-    """V (K,), dQ (K,4), dT (K,3); the kernels write every row of what they compute."""
-    new = torch.empty if need_grad else torch.zeros
-    return (torch.empty(K, dtype=_f32, device=dev), new(K, 4, dtype=_f32, device=dev),
-            new(K, 3, dtype=_f32, device=dev))
+    """V (K,), dQ (K,4), dT (K,3); the kernels write every row of what they compute.  Gradients that
+    are not computed are zero, from one fill: two cost a value-only evaluation of a few poses as
+    much as its kernel."""
+    V = torch.empty(K, dtype=_f32, device=dev)
+    if need_grad:
+        return (V, torch.empty(K, 4, dtype=_f32, device=dev),
+                torch.empty(K, 3, dtype=_f32, device=dev))
+    zero = torch.zeros(7 * K, dtype=_f32, device=dev)
+    return V, zero[:4 * K].view(K, 4), zero[4 * K:].view(K, 3)
 
 
 def overlap_score_grad_se3_batch(A, B, q, t, *, alpha: float = 0.81, N_real=None, M_real=None,
