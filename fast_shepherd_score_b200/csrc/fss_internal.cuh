@@ -14,7 +14,7 @@ namespace fss {
 // Hard limit of points (or pharmacophore features) per molecule that the fused kernels
 // stage in shared memory.  4096 float4 points = 64 KB per cloud.
 constexpr int kMaxPoints = 4096;
-constexpr int kSmallPoints = 64;   // clouds that fss_score_small.cu scores with a warp a pair
+constexpr int kSmallPoints = 64;   // clouds that fss_score_small.cu can score with a warp a pair
 constexpr int kWidePoints = 512;   // and with a CTA a pair
 
 // Thread-local error message + status helpers (fss_capi.cu).
@@ -184,7 +184,7 @@ PharmTables make_pharm_tables(bool directional);
 
 int num_sms();
 
-// fss_score_small.cu: packed scores of clouds of at most kSmallPoints points; unit_fit may be null
+// fss_score_small.cu: packed scores of clouds of at most kWidePoints points; unit_fit may be null
 int score_small_launch(const float* ref_pts, const int32_t* ref_off, const float* fit_pts,
                        const int32_t* fit_off, const int32_t* pair_ref, const int32_t* pair_fit,
                        int P, int maxN, int maxM, float nk, float ne, float Kc, float aKc,

@@ -1,6 +1,6 @@
 // fss_score_small.cu -- Tanimoto scores of packed pairs of clouds of at most kWidePoints points, with
 // the fit side's gradient of the score in the same pass: a warp for a run of pairs up to
-// kSmallPoints (atom clouds), a CTA a pair above (surfaces).
+// kSmallPoints (atom clouds), a CTA a pair above (surfaces) and for few pairs.
 #include <algorithm>
 
 #include "fss_internal.cuh"
@@ -234,8 +234,8 @@ __global__ void __launch_bounds__(32 * kWarps, 4) score_small_kernel(const Small
   }
 }
 
-// A CTA per pair of larger clouds, up to 64 points a warp: the same rows, split over the warps, and
-// the same bound.  Runs of pairs that share the staged reference were 3 % faster at 400 points and
+// A CTA per pair of larger clouds, up to 64 points a warp, and of few pairs: the same rows, split
+// over the warps, and the same bound.  Runs of pairs that share the staged reference were 3 % faster at 400 points and
 // 40 % slower at 310 (four pairs on some CTAs, three on the rest).  Shared memory: 32 bytes a point
 // of both clouds.  One B200, 1000 charged pairs, before (the Gaussians again in the backward) ->
 // after, forward and backward: 100-400 points 161 + 165 -> 186 + 4 us, 100-210 points 70 + 60 ->
@@ -322,7 +322,13 @@ int score_small_launch(const float* ref_pts, const int32_t* ref_off, const float
               0, nk, ne, Kc, aKc, cKc, score, overlaps, reinterpret_cast<float4*>(unit_fit)};
   const auto kern = esp ? (unit_fit ? score_small_kernel<true, true> : score_small_kernel<true, false>)
                         : (unit_fit ? score_small_kernel<false, true> : score_small_kernel<false, false>);
-  if (maxN > kSmallPoints || maxM > kSmallPoints) {
+  // Few pairs of small clouds leave the SMs to a warp each: they take a CTA with a warp for 16 rows (up
+  // to 3 an SM) or 32 (up to 6).  In us, a 60-point query against molecules of 15-60 points, scores
+  // alone, a thread per row / a warp per pair / now: 30 pairs 5.8 / 6.7 / 4.2, 300 pairs 6.2 / 7.0 /
+  // 4.7, 600 pairs 7.1 / 8.0 / 6.2; 1200 pairs 8.7 / 8.8 (7.7 with 32 rows a warp, but forward and
+  // backward of pairs with references of their own 13.7 and 14.5).
+  const bool small = maxN <= kSmallPoints && maxM <= kSmallPoints;
+  if (!small || P <= 6 * sms) {
     const auto wide = esp ? (unit_fit ? score_wide_kernel<true, true> : score_wide_kernel<true, false>)
                           : (unit_fit ? score_wide_kernel<false, true> : score_wide_kernel<false, false>);
     const size_t smem = 2 * sizeof(float4) * (size_t)(((maxN + 3) & ~3) + ((maxM + 3) & ~3));
@@ -330,7 +336,8 @@ int score_small_launch(const float* ref_pts, const int32_t* ref_off, const float
         cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (ce != cudaSuccess)
       return set_error(FSS_ERR_CUDA, std::string("fss_score_fwd: ") + cudaGetErrorString(ce));
-    const int warps = (std::max(maxN, maxM) - 1) / kSmallPoints + 1;
+    const int rows = !small ? kSmallPoints : P <= 3 * sms ? kRowLanes : 2 * kRowLanes;
+    const int warps = (std::max({maxN, maxM, 1}) - 1) / rows + 1;
     wide<<<P, 32 * warps, smem, st>>>(a);
     return check_launch("fss_score_fwd");
   }
