@@ -382,8 +382,8 @@ int launch_kernel(Kern kern, size_t parked, AlignParams prm, int fewest, int cta
                                        cudaGetErrorString(ce));
   if (fewest > 0)
     prm.chunks = choose_chunks(kern, LPP, prm, cta_per_sm, smem_fixed, smem_thread, fewest);
-  const int ppc = (prm.n_starts + prm.chunks - 1) / prm.chunks;
-  const int threads = tile_threads(ppc, LPP);
+  const int threads = tile_threads((prm.n_starts + prm.chunks - 1) / prm.chunks, LPP);
+  const int ppc = threads / LPP;   // poses that a CTA's whole warps hold: what the kernels count by
   prm.chunks = (prm.n_starts + ppc - 1) / ppc;   // every start block non-empty
   prm.n_items = prm.n_pairs * prm.chunks;
   const size_t smem = smem_fixed + smem_thread * threads;
