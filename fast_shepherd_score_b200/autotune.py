@@ -135,7 +135,7 @@ def candidates(mode: str, max_fit: int, n_starts: int, tensor_cores: bool = None
         # wait ~24 % of the time at the per-item barrier (measured on 200-400 point surfaces).
         base = _fewest_idle(lpp, n_starts)
         blocks = [base, 2 * base] + [-(-n_starts // (warps * (32 // lpp))) for warps in (1, 2, 4)]
-        blocks = [c for c in dict.fromkeys(blocks) if c <= n_starts]
+        blocks = list(dict.fromkeys(_launched(c, lpp, n_starts) for c in blocks if c <= n_starts))
         for var in variants:
             if var == 3 and _same_kernel(mode, lpp, max_fit):
                 continue
@@ -158,6 +158,13 @@ def _same_kernel(mode: str, lpp: int, max_fit: int) -> bool:
     """Whether variants 1 and 3 launch one kernel: spread_kernel, which takes only the register tile
     (4 fit points a lane in both) from the variant (launch_align in fss_align_kernel.cuh)."""
     return lpp >= 4 and max_fit <= 16 * lpp and not (mode == "esp" and lpp == 32)
+
+
+def _launched(chunks: int, lpp: int, n_starts: int) -> int:
+    """The start blocks that ``chunks`` runs: a CTA's whole warps hold all the poses they can
+    (launch_kernel in fss_align_kernel.cuh)."""
+    warps = -(-(-(-n_starts // chunks)) * lpp // 32)
+    return -(-n_starts // (warps * 32 // lpp))
 
 
 def _fewest_idle(lpp: int, n_starts: int, max_threads: int = 320) -> int:

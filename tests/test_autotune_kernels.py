@@ -32,7 +32,8 @@ def test_each_kernel_once(mode, max_fit, starts):
         spread = lanes >= 4 and max_fit <= 16 * lanes
         if var == 3 and spread and not (mode == "esp" and lanes == 32):
             var = 1
-        return lanes, c["chunks"], c["cta_per_sm"], var, c.get("accumulate", 0)
+        poses = -(-(-(-starts // c["chunks"]) * lanes) // 32) * 32 // lanes   # of whole warps
+        return lanes, -(-starts // poses), c["cta_per_sm"], var, c.get("accumulate", 0)
     tiles = [kernel(c) for c in autotune.candidates(mode, max_fit, starts, tensor_cores=True)]
     assert len(tiles) == len(set(tiles))
 
