@@ -443,7 +443,11 @@ __device__ __forceinline__ void pose_sums(const ShapeArgs& a, const Rot& R, int 
 //    and ex2, so warps count (8 x 60, 16 lanes, at 168 / 128 / 96 registers: 256 pairs 1.08 / 1.04 /
 //    1.03 ms, 4096 pairs 8.51 / 7.93 / 7.80; align_kernel at 96: 1.10 and 8.08), and
 //    128 for a few pairs (64 pairs, 4 lanes: 2.60 / 2.49 / 2.48);
-//  * two channels, pharmacophores: 128 (16 384 pairs of 20 x 100: 24.8 ms, 25.9 ms at 168);
+//  * two channels: 128 (16 384 pairs of 20 x 100: 24.8 ms, 25.9 ms at 168);
+//  * pharmacophores: 96 from 8 lanes on, where warps hide the feature loops (1000 pairs, 128 / 96
+//    registers: 3-20 features, 32 x 50, 8 lanes 512 / 481 us; 150-300 features, 20 x 30, 8 lanes
+//    15.7 / 12.7 ms, 16 lanes 14.5 / 12.5, align_kernel at 96 13.3 and 13.4), 128 at 4 lanes
+//    (437 / 465 us; 18.1 / 19.9 ms);
 //  * last tiles of up to 5 points, 4 with a second channel beside them: the warps of ragged pairs
 //    run different tiles, and more of them, or longer loops, miss the instruction cache (8192
 //    shape + pharm pairs, 8 lanes: 34.5 ms with up to 4 points unrolled twice, 35.4 unrolled
@@ -459,7 +463,10 @@ struct SpreadTile {
   static constexpr bool kTwo = MODE == FSS_MODE_SHAPE_PHARM || MODE == FSS_MODE_SHAPE_COLOR ||
                                MODE == FSS_MODE_PHARM;
   static constexpr int kRegs =
-      kTwo ? 128 : MODE != FSS_MODE_ESP_COMBO ? 168 : ALONE ? 128 : 96;
+      MODE == FSS_MODE_PHARM ? (LPP >= 8 ? 96 : 128)
+      : kTwo ? 128
+      : MODE != FSS_MODE_ESP_COMBO ? 168
+      : ALONE ? 128 : 96;
   static constexpr int kTail = GROUP == 8 || ALONE ? 8 : kTwo || MODE == FSS_MODE_ESP_COMBO ? 4 : 5;
   static constexpr int kUnroll = kTwo || GROUP == 8 ? 2 : 4;
   static constexpr int kFarUnroll = LPP <= (kTwo ? 4 : 8) && !ALONE ? 1 : 2;
