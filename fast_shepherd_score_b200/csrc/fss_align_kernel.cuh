@@ -404,9 +404,9 @@ __global__ void spread_kernel(const AlignParams p);
 // one is taken: spread_kernel from 4 lanes a pose on, where a lane has at most 16 fit points --
 // beyond that the pairwise loop hides the optimiser, and align_kernel's tiles of four are the
 // better loop (256 surfaces of 200-400 points, 16 lanes: 83.4 and 86.1 ms; 8 lanes, shape: 23.7
-// and 25.8 ms; 256 pairs of 15-50 atoms, 8 lanes: 1.77 and 1.56 ms).  align_kernel also keeps
-// the tensor-core paths and the variants whose rounding of the rotation is their own: 2 and 4,
-// and 1 for ESP at 32 lanes.
+// and 25.8 ms; 256 pairs of 15-50 atoms, 8 lanes: 1.77 and 1.56 ms).  Pharmacophores alone have no
+// such loop and take spread_kernel at any size.  align_kernel also keeps the tensor-core paths and
+// the variants whose rounding of the rotation is their own: 2 and 4, and 1 for ESP at 32 lanes.
 template <int LPP, int MODE, int ACC, int VAR, int EXT = 0>
 int launch_align(const AlignParams& prm, int fewest, int cta_per_sm, size_t smem_fixed,
                  cudaStream_t st) {
@@ -421,12 +421,14 @@ int launch_align(const AlignParams& prm, int fewest, int cta_per_sm, size_t smem
         return launch_kernel<LPP>(spread_kernel<LPP, MODE, kGroup, EXT, true>, 0, prm, fewest,
                                   cta_per_sm, smem_fixed, st);
     }
-    if (prm.maxM <= 16 * LPP)
+    if (MODE == FSS_MODE_PHARM || prm.maxM <= 16 * LPP)
       return launch_kernel<LPP>(spread_kernel<LPP, MODE, kGroup, EXT, false>, 0, prm, fewest,
                                 cta_per_sm, smem_fixed, st);
   }
-  return launch_kernel<LPP>(align_kernel<LPP, MODE, ACC, VAR, EXT>, sizeof(float) * kColdFields,
-                            prm, fewest, cta_per_sm, smem_fixed, st);
+  if constexpr (!kSpread || MODE != FSS_MODE_PHARM)
+    return launch_kernel<LPP>(align_kernel<LPP, MODE, ACC, VAR, EXT>, sizeof(float) * kColdFields,
+                              prm, fewest, cta_per_sm, smem_fixed, st);
+  return set_error(FSS_ERR_UNSUPPORTED, "fss_align: no kernel for this tile");   // not reached
 }
 
 template <int MODE, int VAR, int EXT = 0>
