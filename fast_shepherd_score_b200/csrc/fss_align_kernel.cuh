@@ -407,11 +407,13 @@ __global__ void spread_kernel(const AlignParams p);
 // and 25.8 ms; 256 pairs of 15-50 atoms, 8 lanes: 1.77 and 1.56 ms).  Pharmacophores alone have no
 // such loop and take spread_kernel at any size.  align_kernel also keeps the tensor-core paths and
 // the variants whose rounding of the rotation is their own: 2 and 4, and 1 for ESP at 32 lanes.
+// Builds with another tail or another odd last point (FSS_TAIL_RCP, FSS_PLAIN_TAIL) have only
+// align_kernel: spread_kernel reproduces the default ones.
 template <int LPP, int MODE, int ACC, int VAR, int EXT = 0>
 int launch_align(const AlignParams& prm, int fewest, int cta_per_sm, size_t smem_fixed,
                  cudaStream_t st) {
-  constexpr bool kSpread = LPP >= 4 && ACC == 0 && VAR != 1 && VAR != 3 &&
-                           !(LPP == 32 && MODE == FSS_MODE_ESP && VAR == 0);
+  constexpr bool kSpread = FSS_TAIL_RCP && FSS_PLAIN_TAIL && LPP >= 4 && ACC == 0 && VAR != 1 &&
+                           VAR != 3 && !(LPP == 32 && MODE == FSS_MODE_ESP && VAR == 0);
   if constexpr (kSpread) {
     constexpr int kGroup = 2 * AlignVariant<VAR>::kJB2;
     constexpr bool kOneChannel = MODE == FSS_MODE_SHAPE || MODE == FSS_MODE_ESP ||
