@@ -254,8 +254,9 @@ int overlap_eval_launch(const float* A, const float* B, const float* CA, const f
   // 16.5, 6000 72 and 88; 3000 of 300 points 92 and 77; 13 000 of 400 against 30 points 48.8 and 55.3.
   const bool wide = Mpad > 64 && ((Mpad >= 256 && Npad > 64) || K <= 12 * num_sms());
   // One warp: the loop unrolled twice instead of four times needs fewer registers (more poses on
-  // an SM) and pays for small clouds in large batches: 13 000 poses of 30 points 14.7 and 14.1 us,
-  // charged 17.1 and 16.0; 600 of 50 points 4.9 and 4.7.
+  // an SM) and pays for small clouds in large batches (four times, twice): 13 000 poses of 30 points
+  // 14.7 and 14.1 us,
+  // charged 17.1 and 16.0; 600 of 50 points 4.7 and 4.9.
   const bool few = K <= (esp ? 16 : 24) * num_sms() || Npad > 100;
   const auto kern = esp ? (wide ? overlap_eval_kernel<true, 2, 4>
                            : few ? overlap_eval_kernel<true, 1, 4> : overlap_eval_kernel<true, 1, 2>)

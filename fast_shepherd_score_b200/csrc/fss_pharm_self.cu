@@ -167,7 +167,8 @@ int pharm_self_launch(const float* anc, const float* vec, const int32_t* off, in
   if (max_n > kMaxPoints) return set_error(FSS_ERR_UNSUPPORTED, "fss_pharm_self_overlap: molecule too large");
   if (n_mol == 0) return FSS_OK;
   if (max_n < 0) return set_error(FSS_ERR_INVALID, "fss_pharm_self_overlap: negative extent");
-  // a molecule has to fit the shared memory with anchors and vectors staged twice
+  // An alignment stages the anchors and vectors of both sides: a molecule it could not take against
+  // itself (more than 3631 features) is refused here too, although this kernel stages it once.
   if (4 * sizeof(float4) * (size_t)max_n + 16 > (227u << 10))
     return set_error(FSS_ERR_CUDA, "fss_pharm_self_overlap: molecule too large for shared memory");
   const size_t per = 2 * sizeof(float4) * (size_t)max_n;
