@@ -11,9 +11,14 @@
 //    reference points (pose_tile) instead of running loops of their own: 5 points per lane are
 //    one loop, not one of four points and one of a single point with nothing to overlap.
 //
-// Every rounding on the path is written out (__fmaf_rn and the like), so that a tile's results
-// are the bits align_kernel gave and stay so whatever else changes around them: an alignment
-// amplifies one last bit to another optimum within some thirty steps.
+// A tile's results are the bits align_kernel gives: an alignment amplifies one last bit to another
+// optimum within some thirty steps, and one oversized molecule changes the kernel for all pairs of
+// a launch.  The pairwise sums, the reduction, the rotation and the update of each component have
+// their roundings written out (__fmaf_rn and the like).  The rest is plain arithmetic as in
+// align_kernel: the sums of four products in update, the scores and gradients of combo and
+// esp_combo, and what both kernels share (quat_grad_from_moment, pharm_pose, esp_side).  There the
+// equality rests on the compiler contracting the same expressions alike; it holds for nvcc 12.9 and
+// is what tests/test_gpu_spread.py and test_gpu_spread_far.py compare.
 #pragma once
 #include "fss_align_kernel.cuh"
 
