@@ -95,7 +95,9 @@ def align_packed(mode: str, *, pair_ref, pair_fit, seed_q, seed_t, steps: int, l
     2 tensor-core value/gradient sums, 3 tensor-core exponents (2 and 3: modes "shape" and
     "esp", 32 lanes per pose).  ``kernel_variant`` picks the
     FP32-lane loop's code variant: 0 automatic, 1 base, 2 wide register tile, 3 one-CTA/SM
-    register budget (2 and 3 for "shape" and "esp").  Mode "pharm" only: ``similarity`` in
+    register budget, 4 base tile unrolled 4x, 5 eight-point register tile (2 to 5 for "shape" and
+    "esp", 3 also for "esp_combo"; from 4 lanes per pose and up to 16 fit points per lane 1 and 3
+    are one kernel, except for "esp" at 32 lanes).  Mode "pharm" only: ``similarity`` in
     ("tanimoto", "tversky", "tversky_ref", "tversky_fit") and ``pharm_extended`` 0 (cosine
     weights), 1 (extended points and anchors), 2 (extended points only).
     Mode "esp_combo" (vol_and_surf_esp): ``ref``/``fit`` are the shape centres; ``ref_atoms`` /

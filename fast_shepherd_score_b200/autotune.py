@@ -11,8 +11,9 @@ Tunables of one launch (``fss_align_desc``):
                   32 lanes per pose)
   kernel_variant  code variant of the FP32-lane loop (shape/ESP modes): 1 base, 2 wide
                   register tile, 3 one-CTA/SM register budget, 4 base tile unrolled 4x,
-                  5 eight-point register tile (small molecules); where the optimiser state is
-                  spread over a pose's lanes, 1 and 3 are one kernel and are tried once
+                  5 eight-point register tile (small molecules); from 4 lanes per pose and up to
+                  16 fit points per lane registers and unroll are the kernel's own, and 1 and 3
+                  are one kernel that is tried once (_same_kernel)
 
 For a new problem shape the tuner times each candidate on a sample of the batch's pairs
 (the costliest and a spread of the rest) for a few Adam steps, with CUDA events, and keeps

@@ -62,6 +62,8 @@ constexpr int kMaxThreads = 320;  // 10 warps
 //   4  8 fit points per lane, unrolled 2x, register budget of one 320-thread CTA per SM: one
 //      pass over the reference cloud for every fit cloud of up to 8 x lanes-per-pose points
 //      (small molecules, whose second pass would run mostly empty register tiles)
+// spread_kernel (launch_align says where it runs) takes only the points per lane from the variant;
+// its registers and unroll are SpreadTile's.
 template <int VAR>
 struct AlignVariant;
 template <>

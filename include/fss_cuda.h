@@ -176,7 +176,9 @@ typedef struct fss_align_desc {
                               * CTA/SM register budget), 4 unrolled (4 fit points, 4x unroll,
                               * 2 CTAs/SM budget), 5 small-molecule tile (8 fit points, one
                               * CTA/SM budget); 2-5 for modes SHAPE and ESP, 3 also for
-                              * ESP_COMBO */
+                              * ESP_COMBO.  From 4 lanes per pose and up to 16 fit points per
+                              * lane 1, 3 and 5 choose only the points per lane (1 and 3 are
+                              * one kernel, except 1 for ESP at 32 lanes) */
   int32_t pharm_extended;    /* mode PHARM: 0 cosine-weighted directional features, 1 extended
                               * points (anchor + unit vector) plus anchors, 2 extended points
                               * only (extended_points / only_extended of
