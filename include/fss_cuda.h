@@ -75,7 +75,9 @@ int fss_overlap_grad(const float *A, const float *B, const float *CA, const floa
  * directional = 1 replaces pharm_grad_dq_se3_batch (accel/kernels/pharm_triton.py:403-467);
  * directional = 0 replaces pharm_color_score_grad_se3_batch (pharm_triton.py:254-293,
  * directionless lookup tables).  Types int32 in 0..8 (8 = Dummy, skipped); RV/FV may be NULL
- * when directional == 0. */
+ * when directional == 0.  Up to 32 features a side the order of a pose's sums depends on whether K
+ * exceeds 32 poses an SM: the same call gives the same bits, the pose in a batch of another size
+ * the same value to rounding. */
 int fss_pharm_grad(const float *A, const float *B, const float *RV, const float *FV,
                    const int32_t *At, const int32_t *Bt, const float *q, const float *t,
                    const int32_t *N_real, const int32_t *M_real, int32_t K, int32_t N_pad,
