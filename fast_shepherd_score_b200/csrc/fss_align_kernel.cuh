@@ -315,7 +315,9 @@ inline bool spread_out(const AlignParams& prm, int lpp) {
 //    (starts / pose slots) x (resident warps)^1/4 -- the slots weigh idle lanes; 12 resident
 //    warps instead of 10 (what the staged clouds leave) gave 4 % -- and of equals the smallest,
 //    whose warps wait least for their block's slowest pose (a lane per pose: the largest, which
-//    stages a pair least often).  256 surface pairs, 16 lanes: 104.2 -> 83.4 ms (5-warp ->
+//    stages a pair least often).  Below three rounds a larger CTA has to be 4 % better: its last
+//    round can be nearly empty (256 ESP surface pairs of 50 x 30, 8 lanes: 1-warp CTAs 14.8 ms,
+//    2-warp CTAs in 2.02 rounds 15.4).  256 surface pairs, 16 lanes: 104.2 -> 83.4 ms (5-warp ->
 //    2-warp CTAs); 16 384 shape + pharm pairs of 20 x 100, 8 lanes: 28.1 -> 26.9 ms; 4096 of
 //    50 x 200, 4 lanes: 39.1 -> 32.3 ms.
 template <class Kern>
@@ -340,14 +342,16 @@ int choose_chunks(Kern kern, int lpp, const AlignParams& prm, int cta_per_sm, si
       continue;
     }
     if (cta_per_sm > 0) occ = std::min(occ, cta_per_sm);
-    if ((double)prm.n_pairs * chunks < 2.0 * occ * num_sms()) {
+    const double rounds = (double)prm.n_pairs * chunks / ((double)occ * num_sms());
+    if (rounds < 2.0) {
       if (c == 0) return fewest;
       continue;
     }
     const double score = (double)S * lpp / ((double)chunks * threads) *
                          std::pow((double)occ * (threads / 32), 0.25);
-    if (score > best_score * 1.001 ||
-        (score > best_score * 0.999 && (S + chunks - 1) / chunks < (S + best - 1) / best && lpp > 1)) {
+    const int poses = (S + chunks - 1) / chunks, held = (S + best - 1) / best;
+    if (score > best_score * (poses > held && rounds < 3.0 ? 1.04 : 1.001) ||
+        (score > best_score * 0.999 && poses < held && lpp > 1)) {
       best_score = score;
       best = chunks;
     }
