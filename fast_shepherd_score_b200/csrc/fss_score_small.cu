@@ -283,8 +283,8 @@ __device__ __forceinline__ void wide_pair(const SmallArgs& a, const Cloud A, con
   if (GRAD) write_unit<ESP, R>(a, p, m, first, stride, half, ab, aa, bb, dc, ds);
 }
 
-template <bool ESP, bool GRAD>
-__global__ void __launch_bounds__(32 * kMaxWideWarps, 2) score_wide_kernel(const SmallArgs a) {
+template <bool ESP, bool GRAD, int CTAS>
+__global__ void __launch_bounds__(32 * kMaxWideWarps, CTAS) score_wide_kernel(const SmallArgs a) {
   extern __shared__ __align__(16) float4 smem[];
   __shared__ float red[kMaxWideWarps][3];
   const int pn = (a.maxN + 3) & ~3, pm = (a.maxM + 3) & ~3;
@@ -354,8 +354,15 @@ int score_small_launch(const float* ref_pts, const int32_t* ref_off, const float
     const size_t smem = 2 * sizeof(float4) * (size_t)(((maxN + 3) & ~3) + ((maxM + 3) & ~3));
     const int rows = !small ? kSmallPoints : P <= 3 * sms ? kRowLanes : 2 * kRowLanes;
     const int warps = (std::max({maxN, maxM, 1}) - 1) / rows + 1;
-    const auto wide = esp ? (unit_fit ? score_wide_kernel<true, true> : score_wide_kernel<true, false>)
-                          : (unit_fit ? score_wide_kernel<false, true> : score_wide_kernel<false, false>);
+    // With the gradient, four rows a lane want 128 registers, two CTAs an SM; 80 registers and three
+    // CTAs are faster where a lane has at most two rows or where many CTAs wait.  In us, forward and
+    // backward, 128 and 80 registers (a thread per row): a 400-point reference against 15-60 points,
+    // 300 pairs 39.9 and 36.0 (43.8); 100-400 points, 300 pairs 49.1 and 57.9 (101); 15-60 points and
+    // one molecule of 512, 2000 pairs 39.8 and 45.5 (61), 20 000 pairs 275 and 217 (237).
+    const bool many = maxM <= 2 * kRowLanes * warps || P > 20 * sms;
+    const auto wide = !unit_fit ? (esp ? score_wide_kernel<true, false, 4> : score_wide_kernel<false, false, 4>)
+                      : many    ? (esp ? score_wide_kernel<true, true, 3> : score_wide_kernel<false, true, 3>)
+                                : (esp ? score_wide_kernel<true, true, 2> : score_wide_kernel<false, true, 2>);
     const cudaError_t ce =
         cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (ce != cudaSuccess)
