@@ -38,7 +38,7 @@ _LOADED = False
 LANES = (1, 2, 4, 8, 16, 32)
 # Revision of the kernels behind a tile, part of the key: a cached ranking of other kernels is not
 # used.  Raised whenever a change to them can change which tile is the fastest.
-KERNELS = 2
+KERNELS = 3
 
 
 def _cache_path() -> str:

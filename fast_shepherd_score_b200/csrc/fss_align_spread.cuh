@@ -444,10 +444,11 @@ __device__ __forceinline__ void pose_sums(const ShapeArgs& a, const Rot& R, int 
 //  * shape, ESP: 168 -- with a few rounds of CTAs the largest pair's serial chain of steps decides
 //    the time, and runs faster beside 11 warps than beside 15 (256 pairs of 15-50 atoms, 8 lanes:
 //    1.56 ms, 2.0 ms at 128 registers);
-//  * ESP combo: 96 -- its field points are spread over all lanes and wait for each other's rsqrt
-//    and ex2, so warps count (8 x 60, 16 lanes, at 168 / 128 / 96 registers: 256 pairs 1.08 / 1.04 /
-//    1.03 ms, 4096 pairs 8.51 / 7.93 / 7.80; align_kernel at 96: 1.10 and 8.08), and
-//    128 for a few pairs (64 pairs, 4 lanes: 2.60 / 2.49 / 2.48);
+//  * ESP combo: 128 -- its field points are spread over all lanes and wait for each other's rsqrt
+//    and ex2, so warps count, but 20 of them (96 registers) gain nothing over 16 (calls of 8 x 60,
+//    16 lanes, at 168 / 128 / 96 registers: 64 pairs 1.62 / 1.53 / 1.58 ms, 1024 pairs 3.86 / 3.48
+//    / 3.81, 4096 pairs 12.8 / 12.0 / 11.8; 50 x 60, 512 pairs 10.2 / 9.5 / 10.3; align_kernel
+//    1.75, 3.88, 12.3 and 10.5);
 //  * two channels: 128 (16 384 pairs of 20 x 100: 24.8 ms, 25.9 ms at 168);
 //  * pharmacophores: 96 from 8 lanes on, where warps hide the feature loops (1000 pairs, 128 / 96
 //    registers: 3-20 features, 32 x 50, 8 lanes 512 / 481 us; 150-300 features, 20 x 30, 8 lanes
@@ -469,9 +470,7 @@ struct SpreadTile {
                                MODE == FSS_MODE_PHARM;
   static constexpr int kRegs =
       MODE == FSS_MODE_PHARM ? (LPP >= 8 ? 96 : 128)
-      : kTwo ? 128
-      : MODE != FSS_MODE_ESP_COMBO ? 168
-      : ALONE ? 128 : 96;
+      : kTwo || MODE == FSS_MODE_ESP_COMBO ? 128 : 168;
   static constexpr int kTail = GROUP == 8 || ALONE ? 8 : kTwo || MODE == FSS_MODE_ESP_COMBO ? 4 : 5;
   static constexpr int kUnroll = kTwo || GROUP == 8 ? 2 : 4;
   static constexpr int kFarUnroll = LPP <= (kTwo ? 4 : 8) && !ALONE ? 1 : 2;
