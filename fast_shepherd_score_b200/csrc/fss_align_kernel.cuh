@@ -359,6 +359,22 @@ int choose_chunks(Kern kern, int lpp, const AlignParams& prm, int cta_per_sm, si
   return best;
 }
 
+// Resident CTAs of an SM for a vol_and_surf_esp launch of spread_kernel.  Where all CTAs would be
+// resident at once, some SMs with one more than others, those with more end last; without the
+// extra one, the cheapest pairs follow on the SMs that are done first.  Kept as it was up to four
+// warps an SM (a scheduler each) and where the extra CTAs are many beside two or three an SM.  One
+// B200, calls of 8 x 60, all resident -> evened: 512 pairs, 16 lanes (3.5 CTAs of 4 warps an SM)
+// 2.61 -> 2.26 ms; 640 pairs, 8 lanes (4.3 of 2) 3.61 -> 3.15; 1024 pairs, 8 lanes (6.9) 4.83 ->
+// 4.16; not evened: 400 pairs, 8 lanes (2.7 of 2) 2.93, 3.25 evened; 256 pairs, 8 lanes (3.5 of 1)
+// 2.49, 2.85 evened.
+inline int even_ctas(int items, int warps, int occ) {
+  const int sms = num_sms(), each = items / sms, extra = items - each * sms;
+  if ((long long)items > (long long)occ * sms || each < 2 || extra == 0 ||
+      (long long)items * warps <= 4LL * sms)
+    return occ;
+  return 2 * extra < sms || each >= 4 ? each : occ;
+}
+
 // `fewest` > 0: the start blocks are chosen here (prm.chunks not set yet), `fewest` of them in
 // the fewest-idle-slots tiling; 0: prm.chunks is the caller's.
 // parked: bytes of shared memory per thread beside the staged clouds.
@@ -398,6 +414,7 @@ int launch_kernel(Kern kern, size_t parked, AlignParams prm, int fewest, int cta
   if (ce != cudaSuccess || occ <= 0)
     return set_error(FSS_ERR_UNSUPPORTED, "fss_align: the tile does not fit on an SM");
   if (cta_per_sm > 0) occ = std::min(occ, cta_per_sm);
+  else if (prm.mode == FSS_MODE_ESP_COMBO && parked == 0) occ = even_ctas(prm.n_items, threads / 32, occ);
   const int grid = std::max(1, std::min(prm.n_items, occ * num_sms()));
   kern<<<grid, threads, smem, st>>>(prm);
   return check_launch("fss_align");
