@@ -273,7 +273,9 @@ int fss_fold_centroids(const float *q, const float *t, const int32_t *pair_ref,
  * w = d/d(charge); zero them first -- molecules shared by several pairs accumulate).  Either
  * grad_ref or grad_fit (not both) may be NULL: that side's adjoint is then not computed.
  * esp != 0 adds the charge factor exp(-(c_i-c_j)^2 * inv_lam).  max_*_points bound the
- * molecules' sizes (a larger pair gets a NaN score and no gradient).
+ * molecules' sizes (a larger pair gets a NaN score and no gradient).  The order of a pair's sums
+ * depends on max_*_points and, up to 64, on whether n_pairs exceeds 3 or 6 an SM: the same call
+ * gives the same bits, the pair in a batch of another size the same values to rounding.
  * ------------------------------------------------------------------------------------- */
 int fss_score_fwd(const float *ref_pts, const int32_t *ref_off, const float *fit_pts,
                   const int32_t *fit_off, const int32_t *pair_ref, const int32_t *pair_fit,
