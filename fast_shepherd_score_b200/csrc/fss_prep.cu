@@ -2,8 +2,8 @@
 // cost keys, the centring of pharmacophore sets and the fold of the centroids into the poses.  Each
 // was a chain of elementwise launches (about 110 a call of 1000 pharmacophore pairs, with a hidden
 // synchronisation in two of them) whose host time exceeded the alignment's; each is bound by the
-// latency of one small launch.  One B200, a call of 1000 pharmacophore pairs 1.9 -> 0.65 ms, of one
-// atom pair 1.05 -> 0.93.
+// latency of one small launch.  One B200, with no free-memory query before them either (run_chunked in
+// memory.py), a call of 1000 pharmacophore pairs 2.0 -> 0.63 ms, of one atom pair 1.05 -> 0.93.
 #include <algorithm>
 
 #include "fss_internal.cuh"
