@@ -361,16 +361,15 @@ int choose_chunks(Kern kern, int lpp, const AlignParams& prm, int cta_per_sm, si
 
 // Resident CTAs of an SM for a vol_and_surf_esp launch of spread_kernel.  Where all CTAs would be
 // resident at once, some SMs with one more than others, those with more end last; without the
-// extra one, the cheapest pairs follow on the SMs that are done first.  Kept as it was up to four
-// warps an SM (a scheduler each) and where the extra CTAs are many beside two or three an SM.  One
-// B200, calls of 8 x 60, all resident -> evened: 512 pairs, 16 lanes (3.5 CTAs of 4 warps an SM)
+// extra one, the cheapest pairs follow on the SMs that are done first.  Kept as it was below eight
+// warps an SM, whose time is one pose's latency, and where the extra CTAs are many beside two or
+// three an SM.  One B200, calls of 8 x 60, all resident -> evened: 512 pairs, 16 lanes (3.5 CTAs of 4 warps an SM)
 // 2.61 -> 2.26 ms; 640 pairs, 8 lanes (4.3 of 2) 3.61 -> 3.15; 1024 pairs, 8 lanes (6.9) 4.83 ->
 // 4.16; not evened: 400 pairs, 8 lanes (2.7 of 2) 2.93, 3.25 evened; 256 pairs, 8 lanes (3.5 of 1)
-// 2.49, 2.85 evened.
+// 2.49, 2.85 evened; 1024 pairs of 15-60 atoms, 4 lanes (6.9 of 1) 13.6, 14.5 evened.
 inline int even_ctas(int items, int warps, int occ) {
   const int sms = num_sms(), each = items / sms, extra = items - each * sms;
-  if ((long long)items > (long long)occ * sms || each < 2 || extra == 0 ||
-      (long long)items * warps <= 4LL * sms)
+  if ((long long)items > (long long)occ * sms || each < 2 || extra == 0 || each * warps < 8)
     return occ;
   return 2 * extra < sms || each >= 4 ? each : occ;
 }
